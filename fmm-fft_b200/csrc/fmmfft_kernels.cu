@@ -41,9 +41,11 @@
 
 #include <mutex>
 #include <new>
+#include <type_traits>
 
 #include "fmmfft_internal.h"
 #include "fmmfft_tc.cuh"
+#include "fmmfft_rows.cuh"
 
 #define FMM_CUDA_TRY(call)                                                              \
   do {                                                                                  \
@@ -189,6 +191,10 @@ template <typename R> struct Dev {
   int coarse_grid;  /* blocks of the coarse-tree kernel an SM holds (0: its operators do not fit) */
   int coarse_dbuf;  /* the coarse-tree kernel's operators in two alternating buffers */
   int fuse_s2m;     /* S2M inside the sections pass where tiles hold whole boxes */
+  /* FP64 plans: tree stages and leaf as row contractions on the FP64 matrix instructions
+   * (fmmfft_rows.cuh) and their operators */
+  int rows;
+  R *r_s2m, *r_m2m, *r_m2l, *r_leaf;
   unsigned env_set; /* knobs an environment switch fixed (the autotuner leaves them): bits below */
   int tuned;        /* the knobs come from the autotuner */
 };
@@ -894,6 +900,50 @@ template <class Prob> static void launch_nb(const Prob &pb, int num_sms, int *st
   cudaLaunchKernelEx(&cfg, tc::k_tc_nbr<Prob>, pb, status);
 }
 
+/* An FP64 row contraction (fmmfft_rows.cuh): blocks of 4 warps, each a range of the rows of one
+ * batch, about two blocks per resident slot, so that the operator is staged once per block and the
+ * last wave is short.  A warp takes as many row tiles as its accumulators allow (4 for up to 4 column
+ * tiles, else 2), and one where that would leave half of the SMs idle. */
+constexpr int rows_rt(int NT, int NPAR) { return NT * NPAR <= 4 ? 4 : 2; }
+template <class Prob, int NT, int RT>
+static void launch_rows_as(const Prob &pb, int batches, int nop, int nhw, int num_sms, cudaStream_t st, int pdl) {
+  constexpr int unit = (kRowsThreads / 32) * RT * 8;
+  const size_t smem = sizeof(double) * (size_t)(nop + nhw);
+  long slots = (long)(220 * 1024 / (smem + 1024));
+  slots = num_sms * (slots < 1 ? 1 : slots > 4 ? 4 : slots);
+  long parts = (2 * slots + batches - 1) / batches;
+  const long units = (pb.rows + unit - 1) / unit;
+  if (parts > units) parts = units;
+  const long rows_blk = (units + parts - 1) / parts * unit;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((pb.rows + rows_blk - 1) / rows_blk), (unsigned)batches);
+  cfg.blockDim = dim3(kRowsThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = pdl ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, k_rows_f64<Prob, NT, RT>, pb, rows_blk, nop);
+}
+/* f with the number of column tiles a warp takes at once as a constant */
+template <class F> static void rows_by_nt(int ncol, F f) {
+  const int nt = (ncol + 7) / 8;
+  if (nt == 1) f(std::integral_constant<int, 1>());
+  else if (nt == 2) f(std::integral_constant<int, 2>());
+  else if (nt == 3) f(std::integral_constant<int, 3>());
+  else f(std::integral_constant<int, 4>());
+}
+template <class Prob> static void launch_rows(const Prob &pb, int batches, int nop, int nhw, int num_sms, cudaStream_t st, int pdl) {
+  rows_by_nt(pb.ncol(), [&](auto ntc) {
+    constexpr int NT = decltype(ntc)::value, big = rows_rt(NT, Prob::NPAR);
+    constexpr long unit = (kRowsThreads / 32) * big * 8;
+    if (pb.rows * batches >= 2L * num_sms * unit) launch_rows_as<Prob, NT, big>(pb, batches, nop, nhw, num_sms, st, pdl);
+    else launch_rows_as<Prob, NT, 1>(pb, batches, nop, nhw, num_sms, st, pdl);
+  });
+}
+
 /* First point of each leaf box for the sections whose shifted target leaves its box
  * (sc >= P/2): reference fmmfft.c:771-803 (far) and :839-954 (near).  For sc > P/2 the value
  * comes from box-1 (local expansion evalmh, window box-2..box with the cotsh offsets); for
@@ -1153,6 +1203,129 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 1) k_leaf(const R *_
 #pragma unroll
       for (int t = 0; t < 8; ++t) dst[t] = acc[t];
     }
+  }
+}
+
+/* Leaf stage for wide boxes with few blocks of k_leaf to run (b >= 128; the reference's own b =
+ * 2048): a block computes 128 targets of both planes of one section, 16 groups of 8 targets times
+ * 16 shares of the 3b window points, so that a transform of 2^16 points fills the device.  The
+ * window and the Toeplitz weights pass through shared memory 1024 points at a time; weights lie in
+ * groups of 8 padded by 16 bytes, so the 8-target groups of a warp read different banks.  Each
+ * weight serves the re and im planes: 128 FMAs for 16 (FP64) shared 16-byte loads.  The shares'
+ * sums are added in a fixed order with the far field.  Bound by the FP64 unit (N = 2^16, P = 4, b = 2048:
+ * 604 M FMAs, 36 us at its rate): 72 us there against k_leaf's 494 on 48 blocks; 64 targets a block
+ * measured 80.  Grid (M / 128, P - 1, transforms). */
+constexpr int kWideMin = 128, kWideTgt = 128, kWideSrc = 1024; /* least b; targets, points at a time */
+template <typename R>
+__global__ void __launch_bounds__(256) k_leaf_wide(const R *__restrict__ psi_n, const R *__restrict__ xt,
+                                                   const R *__restrict__ evalmT, const R *__restrict__ evalmh,
+                                                   const R *__restrict__ cot, R *__restrict__ u, long M, long s, int T,
+                                                   int b, int P) {
+  constexpr int PAD = 16 / (int)sizeof(R), GP = 8 + PAD, NW = (kWideSrc + kWideTgt) / 8 * GP;
+  __shared__ __align__(16) R buf[2 * kWideSrc + NW > 4096 ? 2 * kWideSrc + NW : 4096];
+  __shared__ R hred[2][8], hval[2];
+  R *xw = buf, *cw = buf + 2 * kWideSrc;
+  const int sc = (int)blockIdx.y + 1, tid = threadIdx.x;
+  const long tr = blockIdx.z, S1 = P - 1, pl0 = tr * 2 * S1 + 2L * (sc - 1);
+  const long t0 = (long)blockIdx.x * kWideTgt, box = t0 / b, mask = M - 1;
+  const int j0 = (int)(t0 - box * b);
+  const R *xs = xt + (tr * 2 * P + 2L * sc) * M, *ct = cot + (long)(sc - 1) * 4 * b;
+  const bool shifted = 2 * sc >= P && j0 == 0;
+  if (shifted) { /* the box's first point, evaluated in the box before (window box-2 .. box) */
+    R h[2] = {0, 0};
+    for (int q = tid; q < 3 * b; q += 256) {
+      const long m = (box * b - 2L * b + q) & mask;
+      const R w = ct[q];
+      h[0] = fma(xs[m], w, h[0]), h[1] = fma(xs[M + m], w, h[1]);
+    }
+    for (int k = tid; k < T; k += 256) {
+      const R e = evalmh[(long)(sc - 1) * T + k];
+      const long r = ((box - 1) & (s - 1)) * T + k;
+      h[0] = fma(psi_n[pl0 * s * T + r], e, h[0]), h[1] = fma(psi_n[(pl0 + 1) * s * T + r], e, h[1]);
+    }
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+#pragma unroll
+      for (int o = 16; o; o >>= 1) h[p] += __shfl_xor_sync(0xffffffffu, h[p], o);
+      if ((tid & 31) == 0) hred[p][tid >> 5] = h[p];
+    }
+    __syncthreads();
+    if (tid < 2) {
+      R v = 0;
+      for (int w = 0; w < 8; ++w) v += hred[tid][w];
+      hval[tid] = v;
+    }
+  }
+  const int tg = tid & 15, ss = tid >> 4;
+  R acc[2][8];
+#pragma unroll
+  for (int t = 0; t < 8; ++t) acc[0][t] = acc[1][t] = R(0);
+  for (int q0 = 0; q0 < 3 * b; q0 += kWideSrc) {
+    const int qn = 3 * b - q0 < kWideSrc ? 3 * b - q0 : kWideSrc; /* a multiple of 128, as b is */
+    __syncthreads();
+    for (int e = tid; e < qn; e += 256) {
+      const long m = (box * b - b + q0 + e) & mask;
+      xw[e] = xs[m], xw[kWideSrc + e] = xs[M + m];
+    }
+    const R *cs = ct + q0 + b - j0 - kWideTgt; /* weight of (source q0 + q, target j0 + j): cs[q + 128 - j] */
+    for (int e = tid; e < qn + kWideTgt; e += 256) cw[(e >> 3) * GP + (e & 7)] = cs[e];
+    __syncthreads();
+    for (int q = 8 * ss; q < qn; q += 128) {
+      R x0[8], x1[8], w[16];
+      ld8<R>(xw + q, x0);
+      ld8<R>(xw + kWideSrc + q, x1);
+      const R *c = cw + ((q >> 3) + 15 - tg) * GP;
+      ld8<R>(c, w);
+      ld8<R>(c + GP, w + 8);
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+          acc[0][t] = fma(x0[i], w[i - t + 8], acc[0][t]);
+          acc[1][t] = fma(x1[i], w[i - t + 8], acc[1][t]);
+        }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int p = 0; p < 2; ++p)
+#pragma unroll
+    for (int t = 0; t < 8; ++t) buf[(p * 8 + t) * 256 + tid] = acc[p][t];
+  __syncthreads();
+  const int p = tid >> 7, j = tid & 127;
+  R near = 0, far = 0;
+  for (int q = 0; q < 16; ++q) near += buf[(p * 8 + (j & 7)) * 256 + q * 16 + (j >> 3)];
+  const R *ps = psi_n + ((pl0 + p) * s + box) * T, *E = evalmT + (long)(sc - 1) * T * b + j0 + j;
+  for (int k = 0; k < T; ++k) far = fma(ps[k], E[(long)k * b], far);
+  R v = far + near;
+  if (shifted && j == 0) v = 2 * sc > P ? hval[p] : R(0.5) * (v + hval[p]);
+  u[(pl0 + p) * M + t0 + j] = v;
+}
+
+/* S2M of wide boxes (b >= 128) with few rows: a block per row (section, plane, box), the T outputs
+ * times 1024 / T shares of the b samples (T rounded up to a power of two), added in a fixed order.
+ * The row contraction has one block of work there (48 rows of 2048 samples at the reference's N =
+ * 2^16, P = 4, 16 terms: 380 us, this 5). */
+constexpr int kS2mThreads = 1024;
+template <typename R>
+__global__ void __launch_bounds__(kS2mThreads) k_s2m_wide(const R *__restrict__ xt, const R *__restrict__ initch, R *__restrict__ phi_n,
+                                                  long rows, long M, int T, int b, int P) {
+  __shared__ R red[kS2mThreads];
+  const long r = blockIdx.x, z = blockIdx.y;
+  int lt = 0;
+  while ((1 << lt) < T) ++lt;
+  const int t = threadIdx.x & ((1 << lt) - 1), ks = threadIdx.x >> lt, nks = kS2mThreads >> lt;
+  const R *x = xt + (2L * P * z + 2) * M + r * b;
+  R acc = 0;
+  if (t < T)
+#pragma unroll 8
+    for (int k = ks; k < b; k += nks) acc = fma(x[k], initch[(long)k * T + t], acc);
+  red[threadIdx.x] = acc;
+  __syncthreads();
+  if (threadIdx.x < T) {
+    R v = 0;
+    for (int q = 0; q < nks; ++q) v += red[(q << lt) + threadIdx.x];
+    phi_n[(z * rows + r) * T + threadIdx.x] = v;
   }
 }
 
@@ -2190,6 +2363,7 @@ template <typename R> static int tc_upload_ops(Dev<R> *d, const fmm_ops64 *o, ch
   return rc;
 }
 
+constexpr long kRowsMinRows = 1024; /* FP64 plans: the same with the row contractions of fmmfft_rows.cuh */
 constexpr long kCoarseRows = 4096; /* default: tree levels with fewer rows form the coarse tree */
 
 /* Coarse-tree settings of a plan: threshold (FMMFFT_COARSE_ROWS overrides, 0 turns the
@@ -2212,6 +2386,56 @@ template <typename R> static void coarse_setup(Dev<R> *d) {
   if (d->coarse_grid < 1) d->coarse_rows = 0; /* operator too large for shared memory */
 }
 
+/* Values of the FP64 row contractions' operators: S2M, M2M, M2L, leaf, back to back (nl = n - 2). */
+static long rows_nops(long P, long T, long b, long nl) {
+  return b * rows_npad((int)T) + nl * 10 * rows_blk((int)T) + (P - 1) * rows_nleaf((int)T, (int)b);
+}
+
+/* The FP64 row contractions' operators (rows_idx blocks), laid out on the device from the plan's own
+ * tables: element e of an operator block of np columns is (k, c), zero beyond the table. */
+__device__ __forceinline__ void rows_kc(long e, int np, int &k, int &c) {
+  const int lane = (int)(e & 31), q = (int)(e >> 5), nt = np >> 3;
+  k = q / nt * 4 + (lane & 3), c = q % nt * 8 + (lane >> 2);
+}
+__global__ void k_rows_ops(double *__restrict__ out, const double *__restrict__ initch, const double *__restrict__ bm2m,
+                           const double *__restrict__ bm2l, const double *__restrict__ evalmT,
+                           const double *__restrict__ cot, long total, int T, int b, int nl) {
+  const int Tp = rows_kpad(T), Tn = rows_npad(T), bn = rows_npad(b), blk = rows_blk(T), nlf = rows_nleaf(T, b);
+  const long n_s2m = (long)b * Tn, n_m2m = n_s2m + (long)nl * 2 * blk, n_m2l = n_m2m + (long)nl * 8 * blk;
+  for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x) {
+    int k, c;
+    double v = 0;
+    if (e < n_s2m) {
+      rows_kc(e, Tn, k, c);
+      if (c < T) v = initch[k * T + c];
+    } else if (e < n_m2l) { /* T x T blocks: M2M (left, right child), M2L (left child's four, right child's) */
+      const bool up = e < n_m2m;
+      const long q = up ? e - n_s2m : e - n_m2m, g = q / blk;
+      rows_kc(q - g * blk, Tn, k, c);
+      if (k < T && c < T) {
+        if (up) {
+          v = bm2m[((g >> 1) * 2 * T + (g & 1) * T + k) * T + c];
+        } else { /* rows psi, phi[2B-2], phi[2B-1], phi[2B+2], phi[2B+3] of the stacked operator */
+          const int j = (int)(g & 7), right = j >> 2, seg = (j & 3) + ((j & 3) >= (right ? 3 : 2));
+          v = bm2l[((g >> 3) * 5 * T + seg * T + k) * 2 * T + right * T + c];
+        }
+      }
+    } else {
+      const long q = e - n_m2l, z = q / nlf, r = q - z * nlf;
+      if (r < (long)Tp * bn) {
+        rows_kc(r, bn, k, c);
+        if (k < T && c < b) v = evalmT[(z * T + k) * b + c];
+      } else {
+        const long r2 = r - (long)Tp * bn, seg = r2 / ((long)b * bn);
+        rows_kc(r2 - seg * b * bn, bn, k, c);
+        if (c < b) v = cot[z * 4 * b + seg * b + k + b - c];
+      }
+    }
+    out[e] = v;
+  }
+}
+
+static void rows_smem_limits(int T, int b);
 template <typename R>
 static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, char *err, size_t errlen,
                       size_t *dry_bytes = nullptr) {
@@ -2304,6 +2528,12 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
     d->ok_s2m &= (m & 1) != 0, d->ok_m2m &= (m & 2) != 0, d->ok_m2l &= (m & 4) != 0, d->ok_leaf &= (m & 8) != 0;
     d->ok_lnb &= (m & 8) != 0;
   }
+  /* FP64: row contractions on the matrix instructions, unless a switch steers the stage kernels */
+  d->rows = sizeof(R) == 8 && T <= 32 && b >= 8 && b <= 64 && !(d->env_set & (KNOB_COARSE | KNOB_FUSE));
+  /* a small level's row contraction costs 3 to 4 us, less than the same level in the coarse tree from
+   * about 1024 rows (N = 2^20, P = 32, 15 terms, levels from 4096 / 1024 / 256 rows: 150 / 140 / 140 us a
+   * transform; N = 2^17, 24 terms: 96 / 74 / 75) */
+  if (d->rows && d->coarse_rows > kRowsMinRows) d->coarse_rows = kRowsMinRows;
   const long sz_s2m = d->ok_s2m ? (long)d->kp_s2m * d->np_s2m : 0;
   d->tc_s2m_stride16 = 2L * tc::round16(d->kp_s2m) * d->np_s2m;
   d->tc_m2m_stride16 = 2L * tc::round16(d->kp_m2m) * d->np_m2m;
@@ -2368,6 +2598,7 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
   CARVE(wsm2m, ws_m2m_n, float)
   CARVE(wsm2l, ws_m2l_n, float)
   CARVE(wsleaf, ws_leaf_n, float)
+  CARVE(rops, d->rows ? rows_nops(P, T, b, nlev) : 0, R)
 #undef CARVE
   if (dry_bytes) {
     *dry_bytes = off;
@@ -2418,6 +2649,8 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
   d->ws_m2m = (float *)(base + off_wsm2m);
   d->ws_m2l = (float *)(base + off_wsm2l);
   d->ws_leaf = (float *)(base + off_wsleaf);
+  d->r_s2m = (R *)(base + off_rops), d->r_m2m = d->r_s2m + b * rows_npad((int)T);
+  d->r_m2l = d->r_m2m + nlev * 2 * rows_blk((int)T), d->r_leaf = d->r_m2l + nlev * 8 * rows_blk((int)T);
   cudaMemset(d->status, 0, sizeof(int));
   {
     int dev = 0;
@@ -2427,7 +2660,7 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
 
   /* ---- operator layouts (FP64 on the host, rounded once to R) ---- */
   int rc = 0;
-  size_t hn = (size_t)(10 * T * T);
+  size_t hn = (size_t)(10 * T * T * (nlev ? nlev : 1));
   if ((size_t)(S1 * T * b) > hn) hn = (size_t)(S1 * T * b);
   if ((size_t)(2 * P) > hn) hn = (size_t)(2 * P);
   double *h = (double *)malloc(sizeof(double) * (hn + 16));
@@ -2438,34 +2671,34 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
   rc |= upload<R>(&d->btop, h, T * T, err, errlen);
   for (long L = 2; L <= n - 1; ++L) { /* M2M parent level L uses shftfn/fp index L-2 */
     const double *ops = o->levops + (L - 2) * FMM_NLEVOPS * T * T;
+    double *hl = h + (L - 2) * 2 * T * T;
     for (long k = 0; k < T; ++k)
       for (long t = 0; t < T; ++t) {
-        h[k * T + t] = ops[FMM_SHFTFN * T * T + t * T + k];
-        h[(T + k) * T + t] = ops[FMM_SHFTFP * T * T + t * T + k];
+        hl[k * T + t] = ops[FMM_SHFTFN * T * T + t * T + k];
+        hl[(T + k) * T + t] = ops[FMM_SHFTFP * T * T + t * T + k];
       }
-    R *dst = d->bm2m + (L - 2) * 2 * T * T;
-    rc |= upload<R>(&dst, h, 2 * T * T, err, errlen);
   }
+  rc |= upload<R>(&d->bm2m, h, (size_t)(nlev * 2 * T * T), err, errlen);
   for (long l = 3; l <= n; ++l) { /* M2L+L2L child level l uses index l-3 */
     const double *ops = o->levops + (l - 3) * FMM_NLEVOPS * T * T;
 #define OPT(which, t, k) ops[(which) * T * T + (t) * T + (k)]
     const long N2 = 2 * T;
-    for (long i = 0; i < 10 * T * T; ++i) h[i] = 0;
+    double *hl = h + (l - 3) * 10 * T * T;
+    for (long i = 0; i < 10 * T * T; ++i) hl[i] = 0;
     for (long k = 0; k < T; ++k)
       for (long t = 0; t < T; ++t) {
-        h[(0 * T + k) * N2 + t] = OPT(FMM_SHFTLP, t, k);     /* psi parent -> left */
-        h[(0 * T + k) * N2 + T + t] = OPT(FMM_SHFTLN, t, k); /* psi parent -> right */
-        h[(1 * T + k) * N2 + t] = OPT(FMM_FLIP2P, t, k);     /* phi[2B-2] -> left  (c-2) */
-        h[(1 * T + k) * N2 + T + t] = OPT(FMM_FLIP3P, t, k); /* phi[2B-2] -> right (c-3) */
-        h[(2 * T + k) * N2 + T + t] = OPT(FMM_FLIP2P, t, k); /* phi[2B-1] -> right (c-2) */
-        h[(3 * T + k) * N2 + t] = OPT(FMM_FLIP2N, t, k);     /* phi[2B+2] -> left  (c+2) */
-        h[(4 * T + k) * N2 + t] = OPT(FMM_FLIP3N, t, k);     /* phi[2B+3] -> left  (c+3) */
-        h[(4 * T + k) * N2 + T + t] = OPT(FMM_FLIP2N, t, k); /* phi[2B+3] -> right (c+2) */
+        hl[(0 * T + k) * N2 + t] = OPT(FMM_SHFTLP, t, k);     /* psi parent -> left */
+        hl[(0 * T + k) * N2 + T + t] = OPT(FMM_SHFTLN, t, k); /* psi parent -> right */
+        hl[(1 * T + k) * N2 + t] = OPT(FMM_FLIP2P, t, k);     /* phi[2B-2] -> left  (c-2) */
+        hl[(1 * T + k) * N2 + T + t] = OPT(FMM_FLIP3P, t, k); /* phi[2B-2] -> right (c-3) */
+        hl[(2 * T + k) * N2 + T + t] = OPT(FMM_FLIP2P, t, k); /* phi[2B-1] -> right (c-2) */
+        hl[(3 * T + k) * N2 + t] = OPT(FMM_FLIP2N, t, k);     /* phi[2B+2] -> left  (c+2) */
+        hl[(4 * T + k) * N2 + t] = OPT(FMM_FLIP3N, t, k);     /* phi[2B+3] -> left  (c+3) */
+        hl[(4 * T + k) * N2 + T + t] = OPT(FMM_FLIP2N, t, k); /* phi[2B+3] -> right (c+2) */
       }
 #undef OPT
-    R *dst = d->bm2l + (l - 3) * 10 * T * T;
-    rc |= upload<R>(&dst, h, 10 * T * T, err, errlen);
   }
+  rc |= upload<R>(&d->bm2l, h, (size_t)(nlev * 10 * T * T), err, errlen);
   for (long sc = 1; sc < P; ++sc)
     for (long k = 0; k < T; ++k)
       for (long j = 0; j < b; ++j) h[((sc - 1) * T + k) * b + j] = o->evalm[(j * S1 + (sc - 1)) * T + k];
@@ -2497,6 +2730,16 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
   if (d->comp_tw) rc |= upload_lo(d->twM_lo, hm, 2 * M, err, errlen);
   free(hm);
   if (tc && !rc) rc = tc_upload_ops(d, o, err, errlen);
+  if constexpr (sizeof(R) == 8)
+    if (d->rows && !rc) {
+      rows_smem_limits((int)T, (int)b);
+      k_rows_ops<<<2 * d->num_sms, 256>>>(d->r_s2m, d->initch, d->bm2m, d->bm2l, d->evalmT, d->cot,
+                                          rows_nops(P, T, b, nlev), (int)T, (int)b, (int)nlev);
+      if (cudaStreamSynchronize(0) != cudaSuccess) { /* the plan's executes may run on any stream */
+        snprintf(err, errlen, "operator layout: %s", cudaGetErrorString(cudaGetLastError()));
+        rc = 3;
+      }
+    }
   if (rc) {
     cudaFree(pool);
     delete d;
@@ -2581,7 +2824,7 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
   /* 1-2: sections and their sums */
   stage(ST_SECTIONS);
   /* S2M fused into the sections pass when tiles hold whole leaf boxes */
-  const bool s2m_fused = d->tileM % b == 0 && T % 4 == 0 && d->fuse_s2m;
+  const bool s2m_fused = d->tileM % b == 0 && T % 4 == 0 && d->fuse_s2m && !d->rows;
   if (run(ST_SECTIONS)) {
     int TMt = (int)d->tileM;
     size_t sm = sizeof(C) * TMt * (P + 1) + (s2m_fused ? sizeof(R) * b * T : 0);
@@ -2609,8 +2852,22 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
   stage(ST_S2M);
   if (!s2m_fused && run(ST_S2M)) {
     bool done = false;
+    const long rows1 = 2 * S1 * s;
+    R *const phi_n = d->phi + lvl_off(n, S1e, T);
+    if constexpr (sizeof(R) == 8)
+      if (d->rows) {
+        launch_rows(RowsS2M{d->xt, d->r_s2m, phi_n, rows1, M, (int)T, (int)b, (int)P}, nbt,
+                    (int)b * rows_npad((int)T), 0, d->num_sms, st, d->pdl);
+        done = true;
+      }
+    /* wide boxes whose row contraction (128 rows a block) would not fill the device */
+    if (!done && b >= kWideMin && rows1 < 128L * d->num_sms) {
+      k_s2m_wide<R><<<dim3((unsigned)rows1, (unsigned)nbt), kS2mThreads, 0, st>>>(d->xt, d->initch, phi_n, rows1, M, (int)T,
+                                                                          (int)b, (int)P);
+      done = true;
+    }
     if constexpr (sizeof(R) == 4) {
-      if (d->tc && d->ok_s2m && 2 * S1 * s >= d->tc_min_rows) {
+      if (!done && d->tc && d->ok_s2m && rows1 >= d->tc_min_rows) {
         TcS2M q{};
         q.rows = 2 * S1 * s, q.batches = nbt, q.nchunks = 1, q.clen[0] = (int)b, q.coff[0] = 0;
         q.P = (int)P;
@@ -2646,6 +2903,13 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
   const long m2m_stop = (ctl && ctl->m2m_stop) ? ctl->m2m_stop : (coarse ? Lm + 1 : 2);
   for (long L = n - 1; run(ST_M2M) && L >= m2m_stop; --L) {
     bool done = false;
+    if constexpr (sizeof(R) == 8)
+      if (d->rows) {
+        launch_rows(RowsM2M{d->phi + lvl_off(L + 1, S1e, T), d->r_m2m + (L - 2) * 2 * rows_blk((int)T),
+                            d->phi + lvl_off(L, S1e, T), 2 * S1e * (1L << L), (int)T},
+                    1, 2 * rows_blk((int)T), 0, d->num_sms, st, d->pdl);
+        done = true;
+      }
     if constexpr (sizeof(R) == 4) {
       if (d->tc && d->ok_m2m && 2 * S1 * (1L << L) >= d->tc_min_rows) {
         TcM2M q{};
@@ -2695,6 +2959,14 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
   const long m2l_from = (ctl && ctl->m2l_from) ? ctl->m2l_from : (coarse ? Ll + 1 : 3);
   for (long l = m2l_from; run(ST_M2L) && l <= n; ++l) {
     bool done = false;
+    if constexpr (sizeof(R) == 8)
+      if (d->rows) {
+        launch_rows(RowsM2L{d->psi + lvl_off(l - 1, S1e, T), d->phi + lvl_off(l, S1e, T),
+                            d->r_m2l + (l - 3) * 8 * rows_blk((int)T), d->psi + lvl_off(l, S1e, T),
+                            2 * S1e * (1L << (l - 1)), (int)T, (int)(l - 1)},
+                    1, 8 * rows_blk((int)T), 0, d->num_sms, st, d->pdl);
+        done = true;
+      }
     if constexpr (sizeof(R) == 4) {
       if (d->tc && d->ok_m2l && 2 * S1 * (1L << (l - 1)) >= d->tc_min_rows) {
         TcM2L q{};
@@ -2760,7 +3032,17 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
         done = true;
       }
     }
-    if (!done && b % 8 == 0) {
+    bool direct = false; /* the leaf's kernel evaluates the half-shifted first points itself */
+    if constexpr (sizeof(R) == 8)
+      if (d->rows) {
+        launch_rows(RowsLeaf{pb.psi_n, d->xt, d->r_leaf, d->evalmh, d->cot, d->u, 2 * s * nbt, M, s, (int)T, (int)b,
+                             (int)n, (int)P},
+                    (int)S1, rows_nleaf((int)T, (int)b), rows_kpad((int)T) + 3 * (int)b, d->num_sms, st, d->pdl);
+        done = direct = true;
+      }
+    if (direct) {
+      pf.launches[ST_LEAF]++;
+    } else if (!done && b % 8 == 0) {
       /* direct form; it also evaluates the half-shifted first points */
       /* boxes per block: two 8-target groups per thread for FP32, one for FP64 */
       int NB = (int)((sizeof(R) == 4 ? 512 : 256) / (b / 8));
@@ -2770,9 +3052,14 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
       size_t sm = sizeof(R) * ((size_t)(NB + 3) * skew_pitch(b) +
                                (((size_t)(NB + 1) * skew_pitch(T) + 7) & ~(size_t)7) + 8 * b +
                                ((T + 7) & ~7) + (e_in_smem ? (size_t)T * b : 0));
-      dim3 g((unsigned)(s / NB), (unsigned)(2 * S1), (unsigned)nbt);
-      k_leaf<R><<<g, 256, sm, st>>>(pb.psi_n, d->xt, d->evalmT, d->evalmh, d->cot, d->u, M, s,
-                                    (int)T, (int)b, (int)P, NB, e_in_smem);
+      if (b >= kWideMin && s / NB * 2 * S1 < 2 * d->num_sms) { /* too few blocks to fill the device */
+        k_leaf_wide<R><<<dim3((unsigned)(M / kWideTgt), (unsigned)S1, (unsigned)nbt), 256, 0, st>>>(
+            pb.psi_n, d->xt, d->evalmT, d->evalmh, d->cot, d->u, M, s, (int)T, (int)b, (int)P);
+      } else {
+        dim3 g((unsigned)(s / NB), (unsigned)(2 * S1), (unsigned)nbt);
+        k_leaf<R><<<g, 256, sm, st>>>(pb.psi_n, d->xt, d->evalmT, d->evalmh, d->cot, d->u, M, s,
+                                      (int)T, (int)b, (int)P, NB, e_in_smem);
+      }
       pf.launches[ST_LEAF]++;
     } else if (!done) {
       for (int tr = 0; tr < nbt; ++tr) { /* one launch per transform of the batch */
@@ -3085,6 +3372,21 @@ static int set_smem_limits(void) {
   allow_dyn_smem(tc::k_tc_ws<TcLeaf, true>, lim);
   if (dev < FMMK_MAXDEV) done[dev] = 1;
   return 0;
+}
+
+/* The same for the row contractions that a plan of T terms and b points per box launches (only
+ * those: opting a kernel in loads it). */
+template <class Prob> static void allow_rows(int ncol, int maxopt) {
+  rows_by_nt(ncol, [&](auto ntc) {
+    constexpr int NT = decltype(ntc)::value;
+    allow_dyn_smem(k_rows_f64<Prob, NT, 1>, maxopt);
+    allow_dyn_smem(k_rows_f64<Prob, NT, rows_rt(NT, Prob::NPAR)>, maxopt);
+  });
+}
+static void rows_smem_limits(int T, int b) {
+  int dev = 0, lim = 48 * 1024;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  allow_rows<RowsM2L>(T, lim), allow_rows<RowsM2M>(T, lim), allow_rows<RowsS2M>(T, lim), allow_rows<RowsLeaf>(b, lim);
 }
 
 extern "C" int fmmk_device_ok(char *err, size_t errlen) {
