@@ -45,7 +45,6 @@
 
 #include "fmmfft_internal.h"
 #include "fmmfft_tc.cuh"
-#include "fmmfft_rows.cuh"
 
 #define FMM_CUDA_TRY(call)                                                              \
   do {                                                                                  \
@@ -115,6 +114,8 @@ struct Prof {
   int launches[ST_COUNT];
 };
 
+
+struct TreeStage; /* fmmfft_tree.cuh */
 
 template <typename R> struct Dev {
   using C = typename cplx<R>::T;
@@ -194,7 +195,9 @@ template <typename R> struct Dev {
   /* FP64 plans: tree stages and leaf as row contractions on the FP64 matrix instructions
    * (fmmfft_rows.cuh) and their operators */
   int rows;
-  R *r_s2m, *r_m2m, *r_m2l, *r_leaf;
+  int tree;   /* the sections run whole in k_tree */
+  R *tops;    /* operators of the row contractions and of k_tree (TreeOps) */
+  TreeStage *tstages; /* k_tree's stages: with resident operators, with operators in turn */
   unsigned env_set; /* knobs an environment switch fixed (the autotuner leaves them): bits below */
   int tuned;        /* the knobs come from the autotuner */
 };
@@ -270,6 +273,9 @@ __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
       : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
   return d;
 }
+
+#include "fmmfft_rows.cuh"
+#include "fmmfft_tree.cuh"
 
 /* 8 consecutive values into registers (16-byte loads; p 16-byte aligned). */
 template <typename R> __device__ __forceinline__ void ld8(const R *p, R *o) {
@@ -2386,59 +2392,26 @@ template <typename R> static void coarse_setup(Dev<R> *d) {
   if (d->coarse_grid < 1) d->coarse_rows = 0; /* operator too large for shared memory */
 }
 
-/* Values of the FP64 row contractions' operators: S2M, M2M, M2L, leaf, back to back (nl = n - 2). */
-static long rows_nops(long P, long T, long b, long nl) {
-  return b * rows_npad((int)T) + nl * 10 * rows_blk((int)T) + (P - 1) * rows_nleaf((int)T, (int)b);
-}
-
-/* The FP64 row contractions' operators (rows_idx blocks), laid out on the device from the plan's own
- * tables: element e of an operator block of np columns is (k, c), zero beyond the table. */
-__device__ __forceinline__ void rows_kc(long e, int np, int &k, int &c) {
-  const int lane = (int)(e & 31), q = (int)(e >> 5), nt = np >> 3;
-  k = q / nt * 4 + (lane & 3), c = q % nt * 8 + (lane >> 2);
-}
-__global__ void k_rows_ops(double *__restrict__ out, const double *__restrict__ initch, const double *__restrict__ bm2m,
-                           const double *__restrict__ bm2l, const double *__restrict__ evalmT,
-                           const double *__restrict__ cot, long total, int T, int b, int nl) {
-  const int Tp = rows_kpad(T), Tn = rows_npad(T), bn = rows_npad(b), blk = rows_blk(T), nlf = rows_nleaf(T, b);
-  const long n_s2m = (long)b * Tn, n_m2m = n_s2m + (long)nl * 2 * blk, n_m2l = n_m2m + (long)nl * 8 * blk;
-  for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x) {
-    int k, c;
-    double v = 0;
-    if (e < n_s2m) {
-      rows_kc(e, Tn, k, c);
-      if (c < T) v = initch[k * T + c];
-    } else if (e < n_m2l) { /* T x T blocks: M2M (left, right child), M2L (left child's four, right child's) */
-      const bool up = e < n_m2m;
-      const long q = up ? e - n_s2m : e - n_m2m, g = q / blk;
-      rows_kc(q - g * blk, Tn, k, c);
-      if (k < T && c < T) {
-        if (up) {
-          v = bm2m[((g >> 1) * 2 * T + (g & 1) * T + k) * T + c];
-        } else { /* rows psi, phi[2B-2], phi[2B-1], phi[2B+2], phi[2B+3] of the stacked operator */
-          const int j = (int)(g & 7), right = j >> 2, seg = (j & 3) + ((j & 3) >= (right ? 3 : 2));
-          v = bm2l[((g >> 3) * 5 * T + seg * T + k) * 2 * T + right * T + c];
-        }
-      }
-    } else {
-      const long q = e - n_m2l, z = q / nlf, r = q - z * nlf;
-      if (r < (long)Tp * bn) {
-        rows_kc(r, bn, k, c);
-        if (k < T && c < b) v = evalmT[(z * T + k) * b + c];
-      } else {
-        const long r2 = r - (long)Tp * bn, seg = r2 / ((long)b * bn);
-        rows_kc(r2 - seg * b * bn, bn, k, c);
-        if (c < b) v = cot[z * 4 * b + seg * b + k + b - c];
-      }
-    }
-    out[e] = v;
-  }
+/* Whether the plan's sections run whole in one block (k_tree): FP32 plans (split-TF32 and BF16x3 ones
+ * too, whose tree stages are below the tensor cores' row threshold there) up to what shared memory
+ * holds, FP64 ones up to 1024 points a section.  Measured, k_tree against a launch per stage, us a
+ * transform: FP32, 20 terms, P = 64: one of 2^16 39 / 45, 2^18 70 / 92, 16 of 2^16 120 / 322, 4 of 2^18
+ * (split TF32) 127 / 197; FP64, 16 terms: 16 of 2^16 144 / 232, but 16 of 2^17 345 / 308, where the row
+ * contractions fill the device.  The choice depends on the shape alone, so that a transform takes the
+ * same kernel alone and in a batch.  A switch that steers the stage kernels keeps those. */
+constexpr long kTreeMaxF64 = 1024;
+template <typename R> static void tree_setup(Dev<R> *d) {
+  using E = typename TreeEng<R>::E;
+  const int T = (int)d->T, b = (int)d->b, n = (int)d->n;
+  d->tree = b >= 8 && b <= 64 && n <= kTreeMaxLevel && (sizeof(R) == 4 || d->M <= kTreeMaxF64) &&
+            !(d->env_set & (KNOB_COARSE | KNOB_TCMIN | KNOB_FUSE | KNOB_FORM)) && !getenv("FMMFFT_TC_STAGES") &&
+            !getenv("FMMFFT_LEAF_FORM") && tree_smem<E>(T, b, n, 0) <= (size_t)200 * 1024;
 }
 
 static void rows_smem_limits(int T, int b);
 template <typename R>
 static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, char *err, size_t errlen,
-                      size_t *dry_bytes = nullptr) {
+                      size_t *dry_bytes = nullptr, bool shard = false) {
   using C = typename cplx<R>::T;
   Dev<R> *d = new (std::nothrow) Dev<R>();
   if (!d) return 2;
@@ -2530,6 +2503,9 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
   }
   /* FP64: row contractions on the matrix instructions, unless a switch steers the stage kernels */
   d->rows = sizeof(R) == 8 && T <= 32 && b >= 8 && b <= 64 && !(d->env_set & (KNOB_COARSE | KNOB_FUSE));
+  using E = typename TreeEng<R>::E;
+  if (!shard) tree_setup<R>(d); /* a shard runs its stages in pieces */
+  if (d->tree) d->ok_s2m = d->ok_m2m = d->ok_m2l = d->ok_leaf = d->ok_lnb = 0; /* no stage reaches them */
   /* a small level's row contraction costs 3 to 4 us, less than the same level in the coarse tree from
    * about 1024 rows (N = 2^20, P = 32, 15 terms, levels from 4096 / 1024 / 256 rows: 150 / 140 / 140 us a
    * transform; N = 2^17, 24 terms: 96 / 74 / 75) */
@@ -2598,7 +2574,8 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
   CARVE(wsm2m, ws_m2m_n, float)
   CARVE(wsm2l, ws_m2l_n, float)
   CARVE(wsleaf, ws_leaf_n, float)
-  CARVE(rops, d->rows ? rows_nops(P, T, b, nlev) : 0, R)
+  CARVE(tstages, d->tree ? 2 * kTreeStages : 0, TreeStage)
+  CARVE(tops, d->rows || d->tree ? tree_nops<E>(P, T, b, nlev) : 0, R)
 #undef CARVE
   if (dry_bytes) {
     *dry_bytes = off;
@@ -2649,8 +2626,7 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
   d->ws_m2m = (float *)(base + off_wsm2m);
   d->ws_m2l = (float *)(base + off_wsm2l);
   d->ws_leaf = (float *)(base + off_wsleaf);
-  d->r_s2m = (R *)(base + off_rops), d->r_m2m = d->r_s2m + b * rows_npad((int)T);
-  d->r_m2l = d->r_m2m + nlev * 2 * rows_blk((int)T), d->r_leaf = d->r_m2l + nlev * 8 * rows_blk((int)T);
+  d->tops = (R *)(base + off_tops), d->tstages = (TreeStage *)(base + off_tstages);
   cudaMemset(d->status, 0, sizeof(int));
   {
     int dev = 0;
@@ -2730,16 +2706,20 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
   if (d->comp_tw) rc |= upload_lo(d->twM_lo, hm, 2 * M, err, errlen);
   free(hm);
   if (tc && !rc) rc = tc_upload_ops(d, o, err, errlen);
-  if constexpr (sizeof(R) == 8)
-    if (d->rows && !rc) {
-      rows_smem_limits((int)T, (int)b);
-      k_rows_ops<<<2 * d->num_sms, 256>>>(d->r_s2m, d->initch, d->bm2m, d->bm2l, d->evalmT, d->cot,
-                                          rows_nops(P, T, b, nlev), (int)T, (int)b, (int)nlev);
-      if (cudaStreamSynchronize(0) != cudaSuccess) { /* the plan's executes may run on any stream */
-        snprintf(err, errlen, "operator layout: %s", cudaGetErrorString(cudaGetLastError()));
-        rc = 3;
-      }
+  if ((d->rows || d->tree) && !rc) {
+    if (d->rows) rows_smem_limits((int)T, (int)b);
+    if (d->tree) {
+      TreeStage hs[2 * kTreeStages];
+      tree_stages<E>(hs, (int)T, (int)b, (int)n, 1), tree_stages<E>(hs + kTreeStages, (int)T, (int)b, (int)n, 0);
+      if (cudaMemcpy(d->tstages, hs, sizeof hs, cudaMemcpyHostToDevice) != cudaSuccess) rc = 3;
     }
+    k_tree_ops<E><<<2 * d->num_sms, 256>>>(d->tops, d->initch, d->bm2m, d->bm2l, d->btop, d->evalmT, d->cot,
+                                           tree_nops<E>(P, T, b, nlev), (int)T, (int)b, (int)nlev);
+    if (cudaStreamSynchronize(0) != cudaSuccess) { /* the plan's executes may run on any stream */
+      snprintf(err, errlen, "operator layout: %s", cudaGetErrorString(cudaGetLastError()));
+      rc = 3;
+    }
+  }
   if (rc) {
     cudaFree(pool);
     delete d;
@@ -2821,6 +2801,25 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
     cur = id;
   };
   for (int k = 0; k < ST_COUNT; ++k) pf.launches[k] = 0;
+  bool sums_forked = false;
+  TreeOps<typename TreeEng<R>::E> rop{};
+  rop.set(d->tops, (int)T, (int)b, (int)(n > 2 ? n - 2 : 0));
+  if (d->tree && !ctl) { /* 1-7 in one launch, a block per section */
+    using E = typename TreeEng<R>::E;
+    stage(ST_SECTIONS);
+    /* blocks enough to fill the device: large tiles, small blocks and one operator at a time; else all
+     * operators copied at the start and small tiles on more threads */
+    const bool many = P * nbt > 2L * d->num_sms;
+    const int resident = !many && tree_smem<E>((int)T, (int)b, (int)n, 1) <= (size_t)200 * 1024;
+    const TreeArgs<E> ta{x, d->xt, d->ssum, d->phi, d->psi, d->u, rop, d->evalmh, d->cot,
+                         d->tstages + (resident ? 0 : kTreeStages), M, S1e, (int)P, (int)T, (int)b, (int)n, inverse,
+                         resident, many ? 16 : 256, xin};
+    const dim3 g((unsigned)P, (unsigned)nbt);
+    const size_t sm = tree_smem<E>((int)T, (int)b, (int)n, resident);
+    if (many) k_tree<E, 128><<<g, 128, sm, st>>>(ta);
+    else k_tree<E, 512><<<g, 512, sm, st>>>(ta);
+    pf.launches[ST_SECTIONS]++;
+  } else {
   /* 1-2: sections and their sums */
   stage(ST_SECTIONS);
   /* S2M fused into the sections pass when tiles hold whole leaf boxes */
@@ -2834,7 +2833,6 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
     pf.launches[ST_SECTIONS]++;
   }
   stage(ST_SUMS);
-  bool sums_forked = false;
   if (run(ST_SUMS)) { /* a shard sums its own tiles only */
     const long t0 = ctl ? ctl->sum_t0 : 0, nt = ctl ? ctl->sum_nt : d->ntile;
     C *out = (ctl && ctl->sum_out) ? (C *)ctl->sum_out : d->ssum;
@@ -2856,7 +2854,7 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
     R *const phi_n = d->phi + lvl_off(n, S1e, T);
     if constexpr (sizeof(R) == 8)
       if (d->rows) {
-        launch_rows(RowsS2M{d->xt, d->r_s2m, phi_n, rows1, M, (int)T, (int)b, (int)P}, nbt,
+        launch_rows(RowsS2M{d->xt, rop.s2m, phi_n, rows1, M, (int)T, (int)b, (int)P}, nbt,
                     (int)b * rows_npad((int)T), 0, d->num_sms, st, d->pdl);
         done = true;
       }
@@ -2905,7 +2903,7 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
     bool done = false;
     if constexpr (sizeof(R) == 8)
       if (d->rows) {
-        launch_rows(RowsM2M{d->phi + lvl_off(L + 1, S1e, T), d->r_m2m + (L - 2) * 2 * rows_blk((int)T),
+        launch_rows(RowsM2M{d->phi + lvl_off(L + 1, S1e, T), rop.m2m + (L - 2) * 2 * rows_blk((int)T),
                             d->phi + lvl_off(L, S1e, T), 2 * S1e * (1L << L), (int)T},
                     1, 2 * rows_blk((int)T), 0, d->num_sms, st, d->pdl);
         done = true;
@@ -2962,7 +2960,7 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
     if constexpr (sizeof(R) == 8)
       if (d->rows) {
         launch_rows(RowsM2L{d->psi + lvl_off(l - 1, S1e, T), d->phi + lvl_off(l, S1e, T),
-                            d->r_m2l + (l - 3) * 8 * rows_blk((int)T), d->psi + lvl_off(l, S1e, T),
+                            rop.m2l + (l - 3) * 8 * rows_blk((int)T), d->psi + lvl_off(l, S1e, T),
                             2 * S1e * (1L << (l - 1)), (int)T, (int)(l - 1)},
                     1, 8 * rows_blk((int)T), 0, d->num_sms, st, d->pdl);
         done = true;
@@ -3035,7 +3033,7 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
     bool direct = false; /* the leaf's kernel evaluates the half-shifted first points itself */
     if constexpr (sizeof(R) == 8)
       if (d->rows) {
-        launch_rows(RowsLeaf{pb.psi_n, d->xt, d->r_leaf, d->evalmh, d->cot, d->u, 2 * s * nbt, M, s, (int)T, (int)b,
+        launch_rows(RowsLeaf{pb.psi_n, d->xt, rop.leaf, d->evalmh, d->cot, d->u, 2 * s * nbt, M, s, (int)T, (int)b,
                              (int)n, (int)P},
                     (int)S1, rows_nleaf((int)T, (int)b), rows_kpad((int)T) + 3 * (int)b, d->num_sms, st, d->pdl);
         done = direct = true;
@@ -3080,6 +3078,7 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
       k_leaf_mid<R><<<dim3((unsigned)((2 * s + 255) / 256), (unsigned)nbt), 256, 0, st>>>(
           d->u, d->leaf_fix, M, s, (int)n, (int)b, (int)P);
     }
+  }
   }
   /* 8: combine -> z[P][M] */
   stage(ST_COMBINE);
@@ -3275,19 +3274,19 @@ static int dev_autotune(Dev<R> *d, char *err, size_t errlen) {
     cur = keep;
     tune_apply(d, cur);
   };
-  if (d->tc && !d->bf16) { /* tensor-core kernel: per-stage row forms, 16-lane everywhere, warp-specialised */
+  if (d->tc && !d->bf16 && !d->tree) { /* tensor-core kernel: per-stage row forms, 16-lane everywhere, warp-specialised */
     const long v[] = {-1, 3, 4};
     knob(KNOB_FORM, [](TuneVal &c, long x) { c.tc_form = (int)x; }, v, 3);
   }
-  if (d->tc) {
+  if (d->tc && !d->tree) {
     const long v[] = {1024, 4096, 16384};
     knob(KNOB_TCMIN, [](TuneVal &c, long x) { c.tc_min_rows = x; }, v, 3);
   }
-  if (d->coarse_grid >= 1) {
+  if (d->coarse_grid >= 1 && !d->tree) {
     const long v[] = {0, 2048, 4096, 8192, 16384};
     knob(KNOB_COARSE, [](TuneVal &c, long x) { c.coarse_rows = x; }, v, 4);
   }
-  if (d->tileM % d->b == 0 && d->T % 4 == 0) {
+  if (d->tileM % d->b == 0 && d->T % 4 == 0 && !d->tree) {
     const long v[] = {0, 1};
     knob(KNOB_FUSE, [](TuneVal &c, long x) { c.fuse_s2m = (int)x; }, v, 2);
   }
@@ -3353,6 +3352,8 @@ static int set_smem_limits(void) {
   cudaFuncSetAttribute(k_sections<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_leaf<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_leaf<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+  allow_dyn_smem(k_tree<EngF32, 128>, lim), allow_dyn_smem(k_tree<EngF32, 512>, lim);
+  allow_dyn_smem(k_tree<EngF64, 128>, lim), allow_dyn_smem(k_tree<EngF64, 512>, lim);
   allow_dyn_smem(tc::k_tc_rowgemm<TcS2M>, lim);
   allow_dyn_smem(tc::k_tc_rowgemm<TcM2M>, lim);
   allow_dyn_smem(tc::k_tc_rowgemm<TcM2L>, lim);
@@ -3921,11 +3922,11 @@ extern "C" int fmmk_describe(fmmk_state *st, char *buf, size_t len) {
     const char *form = d->tc_form == 0 ? "row" : d->tc_form == 3 ? "row16" : d->tc_form == 4 ? "ws" : "per_stage";
     snprintf(buf, len,
              "fft_threads=%d coarse_rows=%ld tc_min_rows=%ld fuse_s2m=%d tensor_cores=%s tc_form=%s "
-             "leaf_form=%s tuned=%d",
+             "leaf_form=%s%s tuned=%d",
              d->fft_threads, d->coarse_rows, d->tc_min_rows, d->fuse_s2m,
              d->tc ? (d->bf16 ? "bf16x3" : "tf32x3") : "none", form,
-             !d->tc ? "cuda_cores" : (d->ok_lnb && d->tc_form < 0) ? "neighbour_sum" : d->ok_leaf ? "window_rows" : "cuda_cores",
-             d->tuned);
+             !d->tc || d->tree ? "cuda_cores" : (d->ok_lnb && d->tc_form < 0) ? "neighbour_sum" : d->ok_leaf ? "window_rows" : "cuda_cores",
+             d->tree ? " sections=one_block" : "", d->tuned);
   }
   return 0;
 }
@@ -4431,9 +4432,9 @@ static int shard_create(const fmm_ops64 *og, int precision, int G, int g, ShardI
   /* the shard's rows: P/G sections of M points (only its FFT stage runs) */
   fmm_ops64 of = *og;
   of.P = P / G;
-  int rc = dev_create<R>(&ol, precision, 1, &sh->loc, err, errlen);
-  if (!rc) rc = dev_create<R>(&oc, precision, 1, &sh->crs, err, errlen);
-  if (!rc) rc = dev_create<R>(&of, precision, 1, &sh->fft, err, errlen);
+  int rc = dev_create<R>(&ol, precision, 1, &sh->loc, err, errlen, nullptr, true);
+  if (!rc) rc = dev_create<R>(&oc, precision, 1, &sh->crs, err, errlen, nullptr, true);
+  if (!rc) rc = dev_create<R>(&of, precision, 1, &sh->fft, err, errlen, nullptr, true);
   if (rc) {
     shard_free(sh);
     return rc;

@@ -23,6 +23,11 @@ __host__ __device__ __forceinline__ int rows_npad(int N) { return (N + 7) & ~7; 
 __host__ __device__ __forceinline__ int rows_idx(int k, int c, int np) {
   return ((k >> 2) * (np >> 3) + (c >> 3)) * 32 + (c & 7) * 4 + (k & 3);
 }
+/* the (k, c) of element e of a block of np columns */
+__device__ __forceinline__ void rows_kc(long e, int np, int &k, int &c) {
+  const int lane = (int)(e & 31), q = (int)(e >> 5), nt = np >> 3;
+  k = q / nt * 4 + (lane & 3), c = q % nt * 8 + (lane >> 2);
+}
 /* values of a T x T block, of the S2M operator (b x T) and of a section's leaf operator: the blocks of
  * psi (T x b) and of the boxes before, at and after (b x b) */
 __host__ __device__ __forceinline__ int rows_blk(int T) { return rows_kpad(T) * rows_npad(T); }
