@@ -45,6 +45,7 @@
 
 #include "fmmfft_internal.h"
 #include "fmmfft_tc.cuh"
+#include "fmmfft_tcss.cuh"
 
 #define FMM_CUDA_TRY(call)                                                              \
   do {                                                                                  \
@@ -174,6 +175,8 @@ template <typename R> struct Dev {
    * core-matrix layout (tc::ws_b_index), one block per level or section */
   float *ws_s2m, *ws_m2m, *ws_m2l, *ws_leaf;
   long ws_m2m_stride, ws_m2l_stride, ws_leaf_stride;
+  int Tk;           /* K positions of an expansion in the leaf's operator: T rounded up to 8 */
+  int ss_leaf;      /* stages of the leaf's shared-memory form (tc::k_tc_ss), 0: not used */
   int kp_s2m, np_s2m, kp_m2m, np_m2m, kp_m2l, np_m2l, kp_leaf, np_leaf;
   int ok_s2m, ok_m2m, ok_m2l, ok_leaf;
   int kp_lnb, np_lnb, ok_lnb; /* neighbour-sum leaf (tc::k_tc_nbr): the leaf's default form */
@@ -686,6 +689,69 @@ struct TcLeaf : TcBase { /* batch z = section - 1; s is a power of two (log2s) *
   }
 };
 
+/* The same leaf in the shared-memory form (tc::k_tc_ss): a box's expansion and samples once a tile, the
+ * window by row shifts; output rows go through shared memory and are stored, with the FP32 near-field
+ * terms, in whole rows by neighbouring lanes. */
+struct TcLeafSs : TcLeaf {
+  tc::SsMap m;
+  __device__ const float *abase(int a, long r, int z) const {
+    return a ? xt + (plane(r, z) + 2 * (r >> (log2s + 1)) + 2) * M : psi_n + plane(r, z) * s * T;
+  }
+  __device__ void put_side(long r, int z, float v) const { /* column b: the next box's first point */
+    if (2 * (z + 1) < P) return;
+    const long nb = (r + 1) & (s - 1);
+    if (2 * (z + 1) > P) u[plane(r, z) * M + nb * b] = v;
+    else fixbuf[((r >> log2s) << log2s) + nb] = v;
+  }
+  /* The samples that the FP32 terms of a warp's rows need: lane's four columns c of row k = lane / cpr,
+   * + rpi, .. of MMA rows 32 q .. (row m is box 16 (m % 8) + m / 8 of the tile), and the sample before
+   * the row's first.  Up to kSide loads ahead (b <= 32: all of them). */
+  static constexpr int kSide = 8;
+  struct Side {
+    float4 x[kSide];
+    float prev[kSide];
+  };
+  __device__ __forceinline__ void side_at(const float *xp, long bx0, int mm, int c, float4 &x, float &prev) const {
+    const long j0 = (bx0 + 16 * (mm & 7) + (mm >> 3)) * b + c;
+    x = __ldg(reinterpret_cast<const float4 *>(xp + j0));
+    prev = c == 0 ? __ldg(xp + ((j0 - 1) & (M - 1))) : 0.f;
+  }
+  __device__ __forceinline__ void side_load(Side &sd, long r0, int z, int q, int lane) const {
+    const int cpr = b >> 2, lc = __ffs(cpr) - 1, c = 4 * (lane & (cpr - 1)), rpi = 32 >> lc;
+    const float *xp = abase(1, r0, z);
+#pragma unroll
+    for (int i = 0; i < kSide; ++i)
+      if (i < cpr) side_at(xp, r0 & (s - 1), 32 * q + (lane >> lc) + i * rpi, c, sd.x[i], sd.prev[i]);
+  }
+  __device__ __forceinline__ void put_rows(const Side &sd, long r0, int z, int q, int lane, const float *outs) const {
+    const int cpr = b >> 2, lc = __ffs(cpr) - 1, c = 4 * (lane & (cpr - 1)), rpi = 32 >> lc;
+    const float w0 = w01[2 * z], w1 = w01[2 * z + 1];
+    const bool drop = c == 0 && 2 * (z + 1) > P; /* put_side has the first point */
+    const long bx0 = r0 & (s - 1);
+    float *const up = u + plane(r0, z) * M;
+    auto row = [&](int mm, float4 x, float prev) {
+      const float before = __shfl_up_sync(0xffffffffu, x.w, 1);
+      if (c) prev = before;
+      float4 v = *reinterpret_cast<const float4 *>(outs + mm * (b + 4) + c);
+      v.x = fmaf(w0, x.x, fmaf(w1, prev, v.x)), v.y = fmaf(w0, x.y, fmaf(w1, x.x, v.y));
+      v.z = fmaf(w0, x.z, fmaf(w1, x.y, v.z)), v.w = fmaf(w0, x.w, fmaf(w1, x.z, v.w));
+      float *dst = up + (bx0 + 16 * (mm & 7) + (mm >> 3)) * b + c;
+      if (drop) dst[1] = v.y, dst[2] = v.z, dst[3] = v.w;
+      else *reinterpret_cast<float4 *>(dst) = v;
+    };
+#pragma unroll
+    for (int i = 0; i < kSide; ++i)
+      if (i < cpr) row(32 * q + (lane >> lc) + i * rpi, sd.x[i], sd.prev[i]);
+    for (int i = kSide; i < cpr; ++i) {
+      const int mm = 32 * q + (lane >> lc) + i * rpi;
+      float4 x;
+      float prev;
+      side_at(abase(1, r0, z), bx0, mm, c, x, prev);
+      row(mm, x, prev);
+    }
+  }
+};
+
 /* The same leaf in neighbour-sum form (tc::k_tc_nbr): row r = (transform, plane, box B) holds
  * only box B's own data, A = [psi_B (T) | x_B (b)], and the operator of section sc has the
  * column blocks
@@ -883,6 +949,43 @@ static void launch_tc(const Prob &pb0, int num_sms, int *status, cudaStream_t st
     tc::k_tc_rowgemm16<Prob><<<grid, 256, smem, st>>>(pb, status);
   else
     tc::k_tc_rowgemm<Prob><<<grid, 256, smem, st>>>(pb, status);
+}
+
+/* Whether a contraction fits the shared-memory form: stages (2, else 1; 0: it does not fit) for a row of
+ * nch chunks and w staged output floats.  Nine load steps: what a producer's registers hold twice. */
+static int ss_stages(int kpad, int npad, int nch, int w) {
+  if (2 * npad > 256 || tc::ss_prod(nch) > tc::kSMaxProd || tc::ss_steps(nch) > 9) return 0;
+  for (int nst = 2; nst >= 1; --nst)
+    if (tc::ss_smem_bytes(kpad, npad, nch, nst, w) <= (size_t)226 * 1024) return nst;
+  return 0;
+}
+template <class Prob, int NSTEP>
+static void launch_ss_as(const Prob &pb, int grid, size_t smem, int *status, cudaStream_t st, int pdl) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((tc::ss_prod(pb.m.nch) + tc::kSEpi + 1) * 32);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = pdl ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, tc::k_tc_ss<Prob, NSTEP>, pb, status);
+}
+/* f with the number of load steps of a producer warp as a constant */
+template <class F> static void ss_by_steps(int steps, F f) {
+  if (steps <= 4) f(std::integral_constant<int, 4>());
+  else if (steps <= 6) f(std::integral_constant<int, 6>());
+  else f(std::integral_constant<int, 9>());
+}
+template <class Prob> static void launch_ss(const Prob &pb, int num_sms, int *status, cudaStream_t st, int pdl) {
+  const long tiles = pb.rows / tc::kRows * pb.batches;
+  const int grid = (int)(tiles < num_sms ? tiles : num_sms); /* one CTA per SM: most of its shared memory */
+  const size_t smem = tc::ss_smem_bytes(pb.kpad, pb.npad, pb.m.nch, pb.m.nst, pb.b);
+  ss_by_steps(tc::ss_steps(pb.m.nch), [&](auto n) {
+    launch_ss_as<Prob, decltype(n)::value>(pb, grid, smem, status, st, pdl);
+  });
 }
 
 /* The neighbour-sum row form (tc::k_tc_nbr), persistent, two CTAs per SM; launched like the
@@ -2318,17 +2421,17 @@ template <typename R> static int tc_upload_ops(Dev<R> *d, const fmm_ops64 *o, ch
     }
   if (d->ok_leaf && w01)
     for (long sc = 1; sc < P; ++sc) {
-      const int kp = d->kp_leaf, np = d->np_leaf;
+      const int kp = d->kp_leaf, np = d->np_leaf, Tk = d->Tk;
       const double *ct = o->cot + (sc - 1) * 4 * b;
       for (long i = 0; i < (long)kp * np; ++i) v[i] = 0;
       for (long j = 0; j < b; ++j) {
         for (long k = 0; k < T; ++k) v[j * kp + k] = o->evalm[(j * S1 + (sc - 1)) * T + k];
-        for (long q = 0; q < 3 * b; ++q) v[j * kp + T + q] = ct[q + b - j];
-        v[j * kp + T + j + b] = 0, v[j * kp + T + j + b - 1] = 0; /* d = 0, -1: in FP32 */
+        for (long q = 0; q < 3 * b; ++q) v[j * kp + Tk + q] = ct[q + b - j];
+        v[j * kp + Tk + j + b] = 0, v[j * kp + Tk + j + b - 1] = 0; /* d = 0, -1: in FP32 */
       }
       if (2 * sc >= P) { /* column b: the next box's half-shifted first point (TcLeaf) */
         for (long k = 0; k < T; ++k) v[b * kp + k] = o->evalmh[(sc - P / 2) * T + k];
-        for (long q = 0; q < 3 * b; ++q) v[b * kp + T + q] = ct[q];
+        for (long q = 0; q < 3 * b; ++q) v[b * kp + Tk + q] = ct[q];
       }
       rc |= tc_put(d->tc_leaf[0] + (sc - 1) * 2 * d->tc_leaf_stride, d->tc_leaf[1] + (sc - 1) * d->tc_leaf_stride16,
                    d->ws_leaf + (sc - 1) * d->ws_leaf_stride, v, kp, np, err, errlen, d->bf16);
@@ -2409,6 +2512,7 @@ template <typename R> static void tree_setup(Dev<R> *d) {
 }
 
 static void rows_smem_limits(int T, int b);
+static void ss_smem_limits(void);
 template <typename R>
 static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, char *err, size_t errlen,
                       size_t *dry_bytes = nullptr, bool shard = false) {
@@ -2443,8 +2547,9 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
   d->tc = tc;
   d->kp_s2m = up8(b), d->np_s2m = up16(T);
   d->kp_m2m = up8(2 * T), d->np_m2m = up16(T);
+  d->Tk = up8(T); /* the leaf's segments of K start on a K step */
   d->kp_m2l = up8(5 * T), d->np_m2l = up16(2 * T);
-  d->kp_leaf = up8(T + 3 * b), d->np_leaf = up16(b + 1); /* + the half-shifted column */
+  d->kp_leaf = up8(d->Tk + 3 * b), d->np_leaf = up16(b + 1); /* + the half-shifted column */
   d->kp_lnb = up8(T + b), d->np_lnb = up16(3 * b + 3);    /* three blocks + three half-shift columns */
   auto fits = [&](int kp, int np) {
     return tc && (T % 4 == 0) && (b % 4 == 0) && np <= 256 && kp <= 256 &&
@@ -2504,6 +2609,11 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
   /* FP64: row contractions on the matrix instructions, unless a switch steers the stage kernels */
   d->rows = sizeof(R) == 8 && T <= 32 && b >= 8 && b <= 64 && !(d->env_set & (KNOB_COARSE | KNOB_FUSE));
   using E = typename TreeEng<R>::E;
+  /* The leaf's shared-memory form: whole tiles of 128 boxes, unless a switch steers the stage kernels.  It is
+   * the faster one at every size with them (2^20 T20, P64: 31 us -> 24; 2^26 T16, P256: 860 -> 648). */
+  if (tc && !d->bf16 && d->ok_leaf && b % 8 == 0 && s >= tc::kRows && d->tc_form < 0 && !(d->env_set & KNOB_TCMIN) &&
+      !getenv("FMMFFT_TC_STAGES") && !getenv("FMMFFT_LEAF_FORM"))
+    d->ss_leaf = ss_stages(d->kp_leaf, d->np_leaf, (int)(d->Tk + b) / 4, (int)b);
   if (!shard) tree_setup<R>(d); /* a shard runs its stages in pieces */
   if (d->tree) d->ok_s2m = d->ok_m2m = d->ok_m2l = d->ok_leaf = d->ok_lnb = 0; /* no stage reaches them */
   /* a small level's row contraction costs 3 to 4 us, less than the same level in the coarse tree from
@@ -2706,6 +2816,7 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
   if (d->comp_tw) rc |= upload_lo(d->twM_lo, hm, 2 * M, err, errlen);
   free(hm);
   if (tc && !rc) rc = tc_upload_ops(d, o, err, errlen);
+  if (d->ss_leaf && !rc) ss_smem_limits();
   if ((d->rows || d->tree) && !rc) {
     if (d->rows) rows_smem_limits((int)T, (int)b);
     if (d->tree) {
@@ -3002,7 +3113,19 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
     bool done = false;
     if constexpr (sizeof(R) == 4) {
       const bool tc_leaf_rows = d->tc && 2 * s >= (d->tc_min_rows < 256 ? d->tc_min_rows : 256);
-      if (tc_leaf_rows && d->ok_lnb && d->tc_form < 0) { /* neighbour-sum form */
+      if (tc_leaf_rows && d->ss_leaf) { /* shared-memory form */
+        TcLeafSs q{};
+        q.rows = 2 * s * nbt, q.batches = (int)S1;
+        q.kpad = d->kp_leaf, q.npad = d->np_leaf, q.nout = (int)b;
+        q.bimg = d->tc_leaf[0], q.bimg_stride = 2 * d->tc_leaf_stride, q.w01 = d->lnb_w01;
+        q.fixbuf = d->leaf_fix, q.P = (int)P;
+        q.psi_n = pb.psi_n, q.xt = d->xt, q.u = d->u, q.M = M, q.s = s, q.T = (int)T, q.b = (int)b;
+        q.log2s = (int)n;
+        q.m = {{(int)T, (int)b}, {0, d->Tk}, (d->Tk + (int)b) / 4, 4, {0, d->Tk, d->Tk, d->Tk},
+               {d->Tk, (int)b, (int)b, (int)b}, {0, -1, 0, 1}, d->ss_leaf, s};
+        launch_ss(q, d->num_sms, d->status, st, d->pdl);
+        done = true;
+      } else if (tc_leaf_rows && d->ok_lnb && d->tc_form < 0) { /* neighbour-sum form */
         TcLeafNb q{};
         q.rows = 2 * s * nbt, q.batches = (int)S1, q.nchunks = 2;
         q.clen[0] = (int)T, q.clen[1] = (int)b, q.coff[0] = 0, q.coff[1] = (int)T;
@@ -3018,7 +3141,7 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
         TcLeaf q{};
         q.rows = 2 * s * nbt, q.batches = (int)S1, q.nchunks = 4;
         q.clen[0] = (int)T, q.clen[1] = q.clen[2] = q.clen[3] = (int)b;
-        q.coff[0] = 0, q.coff[1] = (int)T, q.coff[2] = (int)(T + b), q.coff[3] = (int)(T + 2 * b);
+        q.coff[0] = 0, q.coff[1] = d->Tk, q.coff[2] = d->Tk + (int)b, q.coff[3] = d->Tk + (int)(2 * b);
         q.kpad = d->kp_leaf, q.npad = d->np_leaf, q.nout = (int)b;
         q.bimg = d->tc_leaf[0], q.bimg_stride = 2 * d->tc_leaf_stride, q.w01 = d->lnb_w01;
         q.bimg16 = d->tc_leaf[1], q.bimg16_stride = d->tc_leaf_stride16;
@@ -3388,6 +3511,13 @@ static void rows_smem_limits(int T, int b) {
   int dev = 0, lim = 48 * 1024;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   allow_rows<RowsM2L>(T, lim), allow_rows<RowsM2M>(T, lim), allow_rows<RowsS2M>(T, lim), allow_rows<RowsLeaf>(b, lim);
+}
+
+static void ss_smem_limits(void) {
+  int dev = 0, lim = 48 * 1024;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  allow_dyn_smem(tc::k_tc_ss<TcLeafSs, 4>, lim), allow_dyn_smem(tc::k_tc_ss<TcLeafSs, 6>, lim);
+  allow_dyn_smem(tc::k_tc_ss<TcLeafSs, 9>, lim);
 }
 
 extern "C" int fmmk_device_ok(char *err, size_t errlen) {
@@ -3925,7 +4055,7 @@ extern "C" int fmmk_describe(fmmk_state *st, char *buf, size_t len) {
              "leaf_form=%s%s tuned=%d",
              d->fft_threads, d->coarse_rows, d->tc_min_rows, d->fuse_s2m,
              d->tc ? (d->bf16 ? "bf16x3" : "tf32x3") : "none", form,
-             !d->tc || d->tree ? "cuda_cores" : (d->ok_lnb && d->tc_form < 0) ? "neighbour_sum" : d->ok_leaf ? "window_rows" : "cuda_cores",
+             !d->tc || d->tree ? "cuda_cores" : d->ss_leaf ? "shared_operands" : (d->ok_lnb && d->tc_form < 0) ? "neighbour_sum" : d->ok_leaf ? "window_rows" : "cuda_cores",
              d->tree ? " sections=one_block" : "", d->tuned);
   }
   return 0;
