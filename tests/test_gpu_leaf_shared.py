@@ -21,7 +21,7 @@ def fm():
 
 # (N, P, T, b): boxes a section N / P / b
 CASES = [(1 << 11, 2, 8, 8), (1 << 13, 2, 12, 32), (1 << 14, 4, 4, 16), (1 << 15, 8, 20, 8), (1 << 17, 32, 28, 32),
-         (1 << 18, 64, 32, 32), (1 << 18, 32, 8, 64), (1 << 18, 16, 16, 64), (1 << 20, 256, 24, 32), (1 << 20, 8, 20, 32)]
+         (1 << 18, 64, 32, 32), (1 << 20, 256, 24, 32), (1 << 20, 8, 20, 32)]
 
 
 @pytest.mark.parametrize("N,P,T,b", CASES)
