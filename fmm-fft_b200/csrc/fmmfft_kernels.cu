@@ -279,6 +279,7 @@ __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
 
 #include "fmmfft_rows.cuh"
 #include "fmmfft_tree.cuh"
+#include "fmmfft_rows32.cuh"
 
 /* 8 consecutive values into registers (16-byte loads; p 16-byte aligned). */
 template <typename R> __device__ __forceinline__ void ld8(const R *p, R *o) {
@@ -1051,6 +1052,38 @@ template <class Prob> static void launch_rows(const Prob &pb, int batches, int n
     if (pb.rows * batches >= 2L * num_sms * unit) launch_rows_as<Prob, NT, big>(pb, batches, nop, nhw, num_sms, st, pdl);
     else launch_rows_as<Prob, NT, 1>(pb, batches, nop, nhw, num_sms, st, pdl);
   });
+}
+
+/* An FP32 row contraction (fmmfft_rows32.cuh): a persistent grid of twice the resident blocks.  Rows a
+ * thread: 8 where that gives every SM three tiles, 4 where it gives one, else 2 (2^20, P = 64, 16 terms,
+ * M2L of 4 levels: 31 us with 8 or 2 only, 27 so; 2^24, 24 terms, all levels: 4 rows 449 us, 8 rows 318). */
+template <class Prob, int RT>
+static void launch_rows32_as(const Prob &pb, int batches, int nop, int nhw, int num_sms, cudaStream_t st, int pdl) {
+  const int ncx = (pb.ncol() + 3) / 4 * Prob::NPAR, R = RT * rows32_nrg(ncx);
+  const size_t smem = sizeof(float) * (size_t)(nop + nhw + (Prob::kLeaf ? R : 0) + pb.smem(R));
+  const long tiles = (pb.rows + R - 1) / R;
+  long slots = (long)(220 * 1024 / (smem + 1024));
+  slots = num_sms * (slots < 1 ? 1 : slots > 4 ? 4 : slots);
+  long parts = (2 * slots + batches - 1) / batches;
+  if (parts > tiles) parts = tiles;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)parts, (unsigned)batches);
+  cfg.blockDim = dim3((unsigned)((rows32_nrg(ncx) * ncx + 31) / 32 * 32));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = pdl ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, k_rows_f32<Prob, RT>, pb, (int)tiles, nop, nhw);
+}
+template <class Prob> static void launch_rows32(const Prob &pb, int batches, int nop, int nhw, int num_sms, cudaStream_t st, int pdl) {
+  const int ncx = (pb.ncol() + 3) / 4 * Prob::NPAR;
+  const long nrg = rows32_nrg(ncx), rows = pb.rows * batches, plane = 1L << pb.lplane();
+  if (rows >= 3L * num_sms * 8 * nrg && 8 * nrg <= plane) launch_rows32_as<Prob, 8>(pb, batches, nop, nhw, num_sms, st, pdl);
+  else if (rows >= 1L * num_sms * 4 * nrg && 4 * nrg <= plane) launch_rows32_as<Prob, 4>(pb, batches, nop, nhw, num_sms, st, pdl);
+  else launch_rows32_as<Prob, 2>(pb, batches, nop, nhw, num_sms, st, pdl);
 }
 
 /* First point of each leaf box for the sections whose shifted target leaves its box
@@ -2472,7 +2505,7 @@ template <typename R> static int tc_upload_ops(Dev<R> *d, const fmm_ops64 *o, ch
   return rc;
 }
 
-constexpr long kRowsMinRows = 1024; /* FP64 plans: the same with the row contractions of fmmfft_rows.cuh */
+constexpr long kRowsMinRows = 1024; /* the same with the row contractions of fmmfft_rows.cuh, fmmfft_rows32.cuh */
 constexpr long kCoarseRows = 4096; /* default: tree levels with fewer rows form the coarse tree */
 
 /* Coarse-tree settings of a plan: threshold (FMMFFT_COARSE_ROWS overrides, 0 turns the
@@ -2512,6 +2545,7 @@ template <typename R> static void tree_setup(Dev<R> *d) {
 }
 
 static void rows_smem_limits(int T, int b);
+static void rows32_smem_limits(void);
 static void ss_smem_limits(void);
 template <typename R>
 static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, char *err, size_t errlen,
@@ -2606,8 +2640,8 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
     d->ok_s2m &= (m & 1) != 0, d->ok_m2m &= (m & 2) != 0, d->ok_m2l &= (m & 4) != 0, d->ok_leaf &= (m & 8) != 0;
     d->ok_lnb &= (m & 8) != 0;
   }
-  /* FP64: row contractions on the matrix instructions, unless a switch steers the stage kernels */
-  d->rows = sizeof(R) == 8 && T <= 32 && b >= 8 && b <= 64 && !(d->env_set & (KNOB_COARSE | KNOB_FUSE));
+  /* row contractions (FP64 on the matrix instructions, FP32 on the CUDA cores), unless a switch steers the stage kernels */
+  d->rows = !tc && T <= 32 && b >= 8 && b <= 64 && !(d->env_set & (KNOB_COARSE | KNOB_FUSE));
   using E = typename TreeEng<R>::E;
   /* The leaf's shared-memory form: whole tiles of 128 boxes, unless a switch steers the stage kernels.  It is
    * the faster one at every size with them (2^20 T20, P64: 31 us -> 24; 2^26 T16, P256: 860 -> 648). */
@@ -2818,7 +2852,7 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
   if (tc && !rc) rc = tc_upload_ops(d, o, err, errlen);
   if (d->ss_leaf && !rc) ss_smem_limits();
   if ((d->rows || d->tree) && !rc) {
-    if (d->rows) rows_smem_limits((int)T, (int)b);
+    if (d->rows) sizeof(R) == 8 ? rows_smem_limits((int)T, (int)b) : rows32_smem_limits();
     if (d->tree) {
       TreeStage hs[2 * kTreeStages];
       tree_stages<E>(hs, (int)T, (int)b, (int)n, 1), tree_stages<E>(hs + kTreeStages, (int)T, (int)b, (int)n, 0);
@@ -2934,7 +2968,7 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
   /* 1-2: sections and their sums */
   stage(ST_SECTIONS);
   /* S2M fused into the sections pass when tiles hold whole leaf boxes */
-  const bool s2m_fused = d->tileM % b == 0 && T % 4 == 0 && d->fuse_s2m && !d->rows;
+  const bool s2m_fused = d->tileM % b == 0 && T % 4 == 0 && d->fuse_s2m && !(d->rows && sizeof(R) == 8);
   if (run(ST_SECTIONS)) {
     int TMt = (int)d->tileM;
     size_t sm = sizeof(C) * TMt * (P + 1) + (s2m_fused ? sizeof(R) * b * T : 0);
@@ -2967,6 +3001,12 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
       if (d->rows) {
         launch_rows(RowsS2M{d->xt, rop.s2m, phi_n, rows1, M, (int)T, (int)b, (int)P}, nbt,
                     (int)b * rows_npad((int)T), 0, d->num_sms, st, d->pdl);
+        done = true;
+      }
+    if constexpr (sizeof(R) == 4)
+      if (d->rows) {
+        launch_rows32(R32S2M{d->xt, rop.s2m, phi_n, rows1, M, (int)T, (int)b, (int)P}, nbt, (int)b * EngF32::npad((int)T), 0,
+                      d->num_sms, st, d->pdl);
         done = true;
       }
     /* wide boxes whose row contraction (128 rows a block) would not fill the device */
@@ -3020,6 +3060,13 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
         done = true;
       }
     if constexpr (sizeof(R) == 4) {
+      if (d->rows) {
+        const int blk = tree_blk<EngF32>((int)T);
+        launch_rows32(R32M2M{d->phi + lvl_off(L + 1, S1e, T), rop.m2m + (L - 2) * 2 * blk, d->phi + lvl_off(L, S1e, T),
+                             2 * S1e * (1L << L), (int)T},
+                      1, 2 * blk, 0, d->num_sms, st, d->pdl);
+        done = true;
+      }
       if (d->tc && d->ok_m2m && 2 * S1 * (1L << L) >= d->tc_min_rows) {
         TcM2M q{};
         q.rows = 2 * S1e * (1L << L), q.batches = 1, q.nchunks = 1, q.clen[0] = (int)(2 * T), q.coff[0] = 0;
@@ -3077,6 +3124,13 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
         done = true;
       }
     if constexpr (sizeof(R) == 4) {
+      if (d->rows) {
+        const int blk = tree_blk<EngF32>((int)T);
+        launch_rows32(R32M2L{d->psi + lvl_off(l - 1, S1e, T), d->phi + lvl_off(l, S1e, T), rop.m2l + (l - 3) * 8 * blk,
+                             d->psi + lvl_off(l, S1e, T), 2 * S1e * (1L << (l - 1)), (int)T, (int)(l - 1)},
+                      1, 8 * blk, 0, d->num_sms, st, d->pdl);
+        done = true;
+      }
       if (d->tc && d->ok_m2l && 2 * S1 * (1L << (l - 1)) >= d->tc_min_rows) {
         TcM2L q{};
         q.rows = 2 * S1e * (1L << (l - 1)), q.batches = 1, q.nchunks = 3;
@@ -3159,6 +3213,13 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
         launch_rows(RowsLeaf{pb.psi_n, d->xt, rop.leaf, d->evalmh, d->cot, d->u, 2 * s * nbt, M, s, (int)T, (int)b,
                              (int)n, (int)P},
                     (int)S1, rows_nleaf((int)T, (int)b), rows_kpad((int)T) + 3 * (int)b, d->num_sms, st, d->pdl);
+        done = direct = true;
+      }
+    if constexpr (sizeof(R) == 4)
+      if (d->rows) {
+        launch_rows32(R32Leaf{pb.psi_n, d->xt, rop.leaf, d->evalmh, d->cot, d->u, 2 * s * nbt, M, s, (int)T, (int)b, (int)n,
+                              (int)P},
+                      (int)S1, tree_nleaf<EngF32>((int)T, (int)b), rows_kpad((int)T) + 3 * (int)b, d->num_sms, st, d->pdl);
         done = direct = true;
       }
     if (direct) {
@@ -3511,6 +3572,16 @@ static void rows_smem_limits(int T, int b) {
   int dev = 0, lim = 48 * 1024;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   allow_rows<RowsM2L>(T, lim), allow_rows<RowsM2M>(T, lim), allow_rows<RowsS2M>(T, lim), allow_rows<RowsLeaf>(b, lim);
+}
+
+template <class Prob> static void allow_rows32(int maxopt) {
+  allow_dyn_smem(k_rows_f32<Prob, 8>, maxopt), allow_dyn_smem(k_rows_f32<Prob, 4>, maxopt);
+  allow_dyn_smem(k_rows_f32<Prob, 2>, maxopt);
+}
+static void rows32_smem_limits(void) {
+  int dev = 0, lim = 48 * 1024;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  allow_rows32<R32M2L>(lim), allow_rows32<R32M2M>(lim), allow_rows32<R32S2M>(lim), allow_rows32<R32Leaf>(lim);
 }
 
 static void ss_smem_limits(void) {
