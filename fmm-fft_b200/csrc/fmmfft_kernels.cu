@@ -1056,7 +1056,7 @@ template <class Prob> static void launch_rows(const Prob &pb, int batches, int n
 
 /* An FP32 row contraction (fmmfft_rows32.cuh): a persistent grid of twice the resident blocks.  Rows a
  * thread: 8 where that gives every SM three tiles, 4 where it gives one, else 2 (2^20, P = 64, 16 terms,
- * M2L of 4 levels: 31 us with 8 or 2 only, 27 so; 2^24, 24 terms, all levels: 4 rows 449 us, 8 rows 318). */
+ * M2L of 4 levels: 31 us with 8 or 2 only, 27 so; 2^24, 24 terms, all levels: 4 rows 449 us, 8 rows 309). */
 template <class Prob, int RT>
 static void launch_rows32_as(const Prob &pb, int batches, int nop, int nhw, int num_sms, cudaStream_t st, int pdl) {
   const int ncx = (pb.ncol() + 3) / 4 * Prob::NPAR, R = RT * rows32_nrg(ncx);
@@ -2641,12 +2641,20 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
     d->ok_lnb &= (m & 8) != 0;
   }
   /* row contractions (FP64 on the matrix instructions, FP32 on the CUDA cores), unless a switch steers the stage kernels */
-  d->rows = !tc && T <= 32 && b >= 8 && b <= 64 && !(d->env_set & (KNOB_COARSE | KNOB_FUSE));
+  const bool steered = (d->env_set & (KNOB_TCMIN | KNOB_FORM)) || getenv("FMMFFT_TC_STAGES") || getenv("FMMFFT_LEAF_FORM");
+  d->rows = T <= 32 && b >= 8 && b <= 64 && !(d->env_set & (KNOB_COARSE | KNOB_FUSE)) && !(tc && steered);
+  /* A few terms make short rows: the tensor cores' 128-row tiles then wait on their operand's way through
+   * registers to tensor memory, and the CUDA cores are faster (us, FP32 rows against split TF32: 2^26, P =
+   * 256, 16 terms: S2M 211 / 299, M2M 226 / 288, M2L 572 / 641; 2^24, P = 64: M2M of 20 terms 109 / 118, of
+   * 24 terms 124 / 112; M2L of 20 terms 270 / 207).  BF16x3 plans keep their tree levels' arithmetic. */
+  if (tc && !d->bf16 && d->rows) {
+    if (T <= 20) d->ok_s2m = d->ok_m2m = 0;
+    if (T <= 16) d->ok_m2l = 0;
+  }
   using E = typename TreeEng<R>::E;
   /* The leaf's shared-memory form: whole tiles of 128 boxes, unless a switch steers the stage kernels.  It is
    * the faster one at every size with them (2^20 T20, P64: 31 us -> 24; 2^26 T16, P256: 860 -> 648). */
-  if (tc && !d->bf16 && d->ok_leaf && b % 8 == 0 && s >= tc::kRows && d->tc_form < 0 && !(d->env_set & KNOB_TCMIN) &&
-      !getenv("FMMFFT_TC_STAGES") && !getenv("FMMFFT_LEAF_FORM"))
+  if (tc && d->ok_leaf && b % 8 == 0 && s >= tc::kRows && !steered)
     d->ss_leaf = ss_stages(d->kp_leaf, d->np_leaf, (int)(d->Tk + b) / 4, (int)b);
   if (!shard) tree_setup<R>(d); /* a shard runs its stages in pieces */
   if (d->tree) d->ok_s2m = d->ok_m2m = d->ok_m2l = d->ok_leaf = d->ok_lnb = 0; /* no stage reaches them */
@@ -3004,7 +3012,7 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
         done = true;
       }
     if constexpr (sizeof(R) == 4)
-      if (d->rows) {
+      if (d->rows && !(d->ok_s2m && rows1 >= d->tc_min_rows)) {
         launch_rows32(R32S2M{d->xt, rop.s2m, phi_n, rows1, M, (int)T, (int)b, (int)P}, nbt, (int)b * EngF32::npad((int)T), 0,
                       d->num_sms, st, d->pdl);
         done = true;
@@ -3060,14 +3068,15 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
         done = true;
       }
     if constexpr (sizeof(R) == 4) {
-      if (d->rows) {
+      const bool on_tc = d->tc && d->ok_m2m && 2 * S1 * (1L << L) >= d->tc_min_rows;
+      if (d->rows && !on_tc) {
         const int blk = tree_blk<EngF32>((int)T);
         launch_rows32(R32M2M{d->phi + lvl_off(L + 1, S1e, T), rop.m2m + (L - 2) * 2 * blk, d->phi + lvl_off(L, S1e, T),
                              2 * S1e * (1L << L), (int)T},
                       1, 2 * blk, 0, d->num_sms, st, d->pdl);
         done = true;
       }
-      if (d->tc && d->ok_m2m && 2 * S1 * (1L << L) >= d->tc_min_rows) {
+      if (on_tc) {
         TcM2M q{};
         q.rows = 2 * S1e * (1L << L), q.batches = 1, q.nchunks = 1, q.clen[0] = (int)(2 * T), q.coff[0] = 0;
         q.kpad = d->kp_m2m, q.npad = d->np_m2m, q.nout = (int)T;
@@ -3124,14 +3133,15 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
         done = true;
       }
     if constexpr (sizeof(R) == 4) {
-      if (d->rows) {
+      const bool on_tc = d->tc && d->ok_m2l && 2 * S1 * (1L << (l - 1)) >= d->tc_min_rows;
+      if (d->rows && !on_tc) {
         const int blk = tree_blk<EngF32>((int)T);
         launch_rows32(R32M2L{d->psi + lvl_off(l - 1, S1e, T), d->phi + lvl_off(l, S1e, T), rop.m2l + (l - 3) * 8 * blk,
                              d->psi + lvl_off(l, S1e, T), 2 * S1e * (1L << (l - 1)), (int)T, (int)(l - 1)},
                       1, 8 * blk, 0, d->num_sms, st, d->pdl);
         done = true;
       }
-      if (d->tc && d->ok_m2l && 2 * S1 * (1L << (l - 1)) >= d->tc_min_rows) {
+      if (on_tc) {
         TcM2L q{};
         q.rows = 2 * S1e * (1L << (l - 1)), q.batches = 1, q.nchunks = 3;
         q.clen[0] = (int)T, q.clen[1] = (int)(2 * T), q.clen[2] = (int)(2 * T);
@@ -3216,7 +3226,7 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
         done = direct = true;
       }
     if constexpr (sizeof(R) == 4)
-      if (d->rows) {
+      if (d->rows && !done) {
         launch_rows32(R32Leaf{pb.psi_n, d->xt, rop.leaf, d->evalmh, d->cot, d->u, 2 * s * nbt, M, s, (int)T, (int)b, (int)n,
                               (int)P},
                       (int)S1, tree_nleaf<EngF32>((int)T, (int)b), rows_kpad((int)T) + 3 * (int)b, d->num_sms, st, d->pdl);
@@ -3462,7 +3472,7 @@ static int dev_autotune(Dev<R> *d, char *err, size_t errlen) {
     const long v[] = {-1, 3, 4};
     knob(KNOB_FORM, [](TuneVal &c, long x) { c.tc_form = (int)x; }, v, 3);
   }
-  if (d->tc && !d->tree) {
+  if (d->tc && !d->bf16 && !d->tree) { /* which levels of a BF16x3 plan are in BF16 is not left to timing */
     const long v[] = {1024, 4096, 16384};
     knob(KNOB_TCMIN, [](TuneVal &c, long x) { c.tc_min_rows = x; }, v, 3);
   }

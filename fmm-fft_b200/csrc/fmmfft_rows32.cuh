@@ -11,7 +11,7 @@
  * wait for the kernel that made the rows, and kept for all of a block's tiles.
  *
  * Measured against the general row kernels, the direct leaf and more levels in the one-warp-a-row
- * coarse tree (us, FP32, b = 32, P = 64): 2^24, 24 terms: M2L 1010 -> 318, M2M 249 -> 123, leaf 353 -> 250;
+ * coarse tree (us, FP32, b = 32, P = 64): 2^24, 24 terms: M2L 1010 -> 309, M2M 249 -> 123, leaf 353 -> 250;
  * 2^20, 20 terms: M2L 64 -> 33, leaf 35 -> 25, coarse levels 57 -> 25, the transform 214 -> 128.  At 2^24
  * the M2L runs at 40% of the FMA rate, the leaf at 43%: 12 warps an SM hide the loads and barriers
  * between tiles only in part; the small levels of 2^20 are bound by their launches (3 to 4 us each).
@@ -202,7 +202,8 @@ __global__ void __launch_bounds__(kRows32Threads, 3) k_rows_f32(const __grid_con
   constexpr bool kOnePlane = RT > 2; /* a tile lies in one plane: its rows are evenly spaced */
   Tile32 t;
   t.lnb = min(pb.lplane(), __ffs(R) - 1), t.nbt = 1 << t.lnb;
-  const int rg = threadIdx.x / ncx, cx = threadIdx.x - rg * ncx, par = cx >= nc, cg = cx - par * nc;
+  /* parities apart: 8 neighbouring lanes read one operator's columns and two or three rows, no bank twice */
+  const int par = (int)threadIdx.x / (nrg * nc), rem = (int)threadIdx.x - par * nrg * nc, rg = rem / nc, cg = rem - rg * nc;
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     t.r0 = (long)tile * R;
     t.valid = pb.rows - t.r0 < R ? (int)(pb.rows - t.r0) : R;
@@ -230,7 +231,7 @@ __global__ void __launch_bounds__(kRows32Threads, 3) k_rows_f32(const __grid_con
         }
         __syncthreads();
       }
-    if (rg >= nrg) continue;
+    if (par >= Prob::NPAR) continue;
     float2 acc[RT][4];
     int o[RT];
 #pragma unroll

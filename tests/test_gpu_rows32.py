@@ -58,3 +58,29 @@ def test_rows_match_oracle_alone_and_in_a_batch(fm, monkeypatch, N, P, T, b):
     got = y.cpu().numpy().astype(np.complex128).reshape(3, N)
     assert ol.rel_l2(got[0], o["y"]) < 1e-6
     assert ol.rel_l2(got[2], ol.forward(xs[2], P, T, b)) < 1e-6
+
+
+@pytest.mark.parametrize("prec,T,tol", [("f32_tc", 8, 1e-6), ("f32_tc", 16, 1e-6), ("f32_tc", 20, 1e-6), ("f32_tc", 24, 1e-6),
+                                        ("bf16x3", 12, 1e-4), ("bf16x3", 24, 1e-4)])
+def test_rows_beside_tensor_core_stages(fm, monkeypatch, prec, T, tol):
+    """Tensor-core plans on both sides of the terms where S2M, M2M and M2L change units, their small levels
+    as row contractions below the tensor cores' and above the coarse tree; the plans' accuracy classes."""
+    import torch
+    monkeypatch.setenv("FMMFFT_AUTOTUNE", "0")
+    N, P, b = 1 << 20, 32, 32
+    xs = [ol.seeded_input(N, 60 + i) for i in range(2)]
+    plan = fm.Plan(N, P, T, b, prec, max_transforms=2)
+    assert "leaf_form=shared_operands" in plan.describe(), plan.describe()
+    x = torch.from_numpy(np.concatenate(xs)).to(torch.complex64).cuda()
+    y, alone = torch.empty_like(x), torch.empty_like(x)
+    s = torch.cuda.current_stream().cuda_stream
+    plan.execute_many_ptr(2, x.data_ptr(), y.data_ptr(), s)
+    for i in (1, 0):
+        plan.execute_ptr(x[i * N:].data_ptr(), alone[i * N:].data_ptr(), s)
+    torch.cuda.synchronize()
+    plan.check()
+    plan.close()
+    assert torch.equal(y, alone)
+    got = y.cpu().numpy().astype(np.complex128).reshape(2, N)
+    for i in range(2):
+        assert ol.rel_l2(got[i], ol.forward(xs[i], P, T, b)) < tol
