@@ -1661,6 +1661,13 @@ __device__ __forceinline__ int fft_swz(int i, int kw) {
   const int R = i >> 4;
   return i ^ (R & 7) ^ ((R & 4) << 1) ^ kw;
 }
+/* fft_swz(i | c) from si = fft_swz(i), for i and c without common bits: the swizzle is linear over XOR.
+ * With c a constant the bits above a 16-element row become an offset of the access, and one XOR is
+ * left for each different low part. */
+__device__ __forceinline__ int fft_at(int si, int c) {
+  const int z = fft_swz(c, 0);
+  return (si ^ (z & 15)) + (z & ~15);
+}
 /* Shared elements of a register pass: exchange buffer, stage twiddles (L - Ns0 <= L used, the
  * region kept at L + L/16 + 1), 4-step twiddle steps [w][9]. */
 __host__ __device__ __forceinline__ size_t fft_smem_elems(int L, int W) {
@@ -1679,6 +1686,7 @@ template <typename R> struct StridedLd { /* in + row irow + g iseq + i istr */
 #pragma unroll
     for (int r = 0; r < 8; ++r) v[r] = sp[r * qs];
   }
+  __device__ __forceinline__ void finish(long, int, int, typename cplx<R>::T (&)[8]) const {}
 };
 
 /* The combine's input: element sc of column m is x_0[m] for sc = 0, else
@@ -1696,25 +1704,31 @@ template <typename R> struct CombineLd {
                                              typename cplx<R>::T (&v)[8]) const {
     const long m = m0 + mc;
     const R *xt = this->xt + row * 2 * P * M, *u = this->u + row * 2 * (P - 1) * M;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const int sc = t + r * q;
+      const R *const p = sc == 0 ? xt : u + (2L * (sc - 1)) * M;
+      v[r].x = p[m], v[r].y = p[M + m];
+    }
+  }
+  /* the section sums and pre-twiddles, of few sections and many columns, come from L1 */
+  __device__ __forceinline__ void finish(long row, int t, int q, typename cplx<R>::T (&v)[8]) const {
     const typename cplx<R>::T *ssum = this->ssum + row * P;
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
       const int sc = t + r * q;
-      if (sc == 0) {
-        v[r].x = xt[m], v[r].y = xt[M + m];
-      } else {
-        const typename cplx<R>::T S = ssum[sc];
-        typename cplx<R>::T a;
-        a.x = u[(2L * (sc - 1)) * M + m] + S.y * invM;
-        a.y = u[(2L * (sc - 1) + 1) * M + m] - S.x * invM;
-        if constexpr (sizeof(R) == 4) {
-          if (pretw_lo) {
-            v[r] = cmul_comp(a, pretw[sc], pretw_lo[sc]);
-            continue;
-          }
+      if (sc == 0) continue;
+      const typename cplx<R>::T S = ssum[sc];
+      typename cplx<R>::T a;
+      a.x = v[r].x + S.y * invM;
+      a.y = v[r].y - S.x * invM;
+      if constexpr (sizeof(R) == 4) {
+        if (pretw_lo) {
+          v[r] = cmul_comp(a, pretw[sc], pretw_lo[sc]);
+          continue;
         }
-        v[r] = cmul(pretw[sc], a);
       }
+      v[r] = cmul(pretw[sc], a);
     }
   }
 };
@@ -1746,6 +1760,14 @@ __global__ void __launch_bounds__(512, sizeof(R) == 4 ? 3 : 1)
   C *twl_lo = twq + 9 * W;       /* COMP: the remainders of twl */
   const int tid = threadIdx.x;
   const unsigned g0 = blockIdx.x * (unsigned)W;
+  int t, w;
+  if (TIN) t = tid & (q - 1), w = tid >> lq;
+  else w = tid & (W - 1), t = tid >> lW;
+  const long row = blockIdx.y;
+  C v[8];
+  /* on their way while the twiddles are staged: one memory latency a block instead of two (the combine,
+   * whose sums and pre-twiddles also come after: 357 us -> 269 at 2^26, P = 256; 75 -> 53 at 2^24, P = 64) */
+  ld(row, g0 + w, t, q, v);
   /* post-twiddle exp(-2 pi i e / T) for e = g * i */
   auto post = [&](unsigned gi) -> C {
     const unsigned e = (gi * fp.twmul) & fp.twmask;
@@ -1774,38 +1796,34 @@ __global__ void __launch_bounds__(512, sizeof(R) == 4 ? 3 : 1)
       return x;
     }
   };
-  int t, w;
-  if (TIN) t = tid & (q - 1), w = tid >> lq;
-  else w = tid & (W - 1), t = tid >> lW;
   const unsigned ostr = (unsigned)fp.ostr;
-  const long row = blockIdx.y;
-  C v[8];
-  ld(row, g0 + w, t, q, v);
+  ld.finish(row, t, q, v);
   C *bw = buf + w * LP;
   const int kw = W == 8 ? (w >> 2) & 1 : 0;
   int Ns, lNs;
+  const int st = fft_swz(t, kw); /* where element t of the sequence lies */
   if (lg % 3 == 0) { /* radix-8 first stage: outputs 8t + r */
     dft8(v);
+    const int s0 = fft_swz(8 * t, kw);
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      bw[fft_swz(8 * t + r, kw)] = v[r];
-    }
+    for (int r = 0; r < 8; ++r) bw[fft_at(s0, r)] = v[r];
     Ns = 8, lNs = 3;
   } else if (lg % 3 == 2) { /* radix 4: butterflies t (v0,2,4,6) and t+q (v1,3,5,7) */
     dft4(v[0], v[2], v[4], v[6]);
     dft4(v[1], v[3], v[5], v[7]);
+    const int s0 = fft_swz(4 * t, kw);
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      bw[fft_swz(4 * t + r, kw)] = v[2 * r];
-      bw[fft_swz(4 * (t + q) + r, kw)] = v[2 * r + 1];
+      bw[fft_at(s0, r)] = v[2 * r];
+      bw[fft_at(s0, 4 * q + r)] = v[2 * r + 1];
     }
     Ns = 4, lNs = 2;
   } else { /* radix 2: butterflies t + m q, inputs v[m], v[m+4] */
+    const int s0 = fft_swz(2 * t, kw);
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
-      const int i = 2 * (t + m * q);
-      bw[fft_swz(i, kw)] = cadd(v[m], v[m + 4]);
-      bw[fft_swz(i + 1, kw)] = csub(v[m], v[m + 4]);
+      bw[fft_at(s0, 2 * m * q)] = cadd(v[m], v[m + 4]);
+      bw[fft_at(s0, 2 * m * q + 1)] = csub(v[m], v[m + 4]);
     }
     Ns = 2, lNs = 1;
   }
@@ -1815,7 +1833,7 @@ __global__ void __launch_bounds__(512, sizeof(R) == 4 ? 3 : 1)
   for (int si = 0; si < nst; ++si) {
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < 8; ++r) v[r] = bw[fft_swz(t + r * q, kw)];
+    for (int r = 0; r < 8; ++r) v[r] = bw[fft_at(st, r * q)];
     const int k = t & (Ns - 1);
     const int tb = Ns - ns0 + 7 * k - 1;
 #pragma unroll
@@ -1828,9 +1846,9 @@ __global__ void __launch_bounds__(512, sizeof(R) == 4 ? 3 : 1)
     dft8(v);
     if (si == nst - 1) break; /* v[r] = output t + r q */
     __syncthreads();
-    const int o = ((t >> lNs) << (lNs + 3)) + k;
+    const int so = fft_swz(((t >> lNs) << (lNs + 3)) + k, kw);
 #pragma unroll
-    for (int r = 0; r < 8; ++r) bw[fft_swz(o + (r << lNs), kw)] = v[r];
+    for (int r = 0; r < 8; ++r) bw[fft_at(so, r << lNs)] = v[r];
     Ns <<= 3, lNs += 3;
   }
   C *dp = ot.rpp ? reinterpret_cast<C *>(ot.p[row / ot.rpp]) + (row % ot.rpp) * fp.orow : out + row * fp.orow;
@@ -1855,7 +1873,7 @@ __global__ void __launch_bounds__(512, sizeof(R) == 4 ? 3 : 1)
   } else {
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < 8; ++r) bw[fft_swz(t + r * q, kw)] = v[r];
+    for (int r = 0; r < 8; ++r) bw[fft_at(st, r * q)] = v[r];
     __syncthreads();
     int t2, w2;
     if (TOUT) t2 = tid & (q - 1), w2 = tid >> lq;
@@ -1867,10 +1885,11 @@ __global__ void __launch_bounds__(512, sizeof(R) == 4 ? 3 : 1)
     const unsigned qs = (unsigned)q * ostr;
     C a;
     if (fp.twiddle_post && !COMP) a = post(g * (unsigned)t2);
+    const int s2 = fft_swz(t2, kw2);
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
       const int i = t2 + r * q;
-      C x = b2[fft_swz(i, kw2)];
+      C x = b2[fft_at(s2, r * q)];
       if (fp.twiddle_post) {
         if constexpr (COMP)
           x = post_comp(x, g * (unsigned)i);
@@ -1881,6 +1900,46 @@ __global__ void __launch_bounds__(512, sizeof(R) == 4 ? 3 : 1)
       op[r * qs] = x;
     }
   }
+}
+
+/* A build for each usual pass length, whose exchange addresses and stage loop are constants but for a few
+ * XORs (2^26, P = 256: the combine 437 us in the build for any L, 357 in its own): f with log2 L as a
+ * constant where it lies in LO .. HI, else 0 */
+template <int LO, int HI, class F> static void fft_by_len(int L, F f) {
+  if constexpr (LO > HI) {
+    f(std::integral_constant<int, 0>());
+  } else {
+    if (L == 1 << LO) f(std::integral_constant<int, LO>());
+    else fft_by_len<LO + 1, HI>(L, f);
+  }
+}
+constexpr int kFftLo = 6, kFftHi = 10, kCombLo = 4, kCombHi = 8;
+template <typename R>
+static void launch_fft_reg(const StridedLd<R> &ld, typename cplx<R>::T *out, const typename cplx<R>::T *twD,
+                           const typename cplx<R>::T *twP, const FftPass &fp, bool tin, bool tout, dim3 g, int thr, size_t sm,
+                           cudaStream_t st, const OutTab &O = OutTab{}) {
+  fft_by_len<kFftLo, kFftHi>(fp.L, [&](auto lgt) {
+    constexpr int G = decltype(lgt)::value;
+    using S = StridedLd<R>;
+    if (tin && tout)
+      k_fft_reg<R, true, true, S, false, G><<<g, thr, sm, st>>>(ld, out, twD, twP, fp, nullptr, nullptr, O);
+    else if (tin)
+      k_fft_reg<R, true, false, S, false, G><<<g, thr, sm, st>>>(ld, out, twD, twP, fp, nullptr, nullptr, O);
+    else
+      k_fft_reg<R, false, false, S, false, G><<<g, thr, sm, st>>>(ld, out, twD, twP, fp, nullptr, nullptr, O);
+  });
+}
+/* the shared-memory opt-in of every build */
+template <typename R, int G, int HI> static void fft_smem_limit(int lim) {
+  constexpr auto at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  if constexpr (G == 0 || (G >= kFftLo && G <= kFftHi)) {
+    cudaFuncSetAttribute(k_fft_reg<R, true, true, StridedLd<R>, false, G>, at, lim);
+    cudaFuncSetAttribute(k_fft_reg<R, true, false, StridedLd<R>, false, G>, at, lim);
+    cudaFuncSetAttribute(k_fft_reg<R, false, false, StridedLd<R>, false, G>, at, lim);
+  }
+  if constexpr (G == 0 || (G >= kCombLo && G <= kCombHi))
+    cudaFuncSetAttribute(k_fft_reg<R, false, false, CombineLd<R>, false, G>, at, lim);
+  if constexpr (G < HI) fft_smem_limit<R, G == 0 ? (kFftLo < kCombLo ? kFftLo : kCombLo) : G + 1, HI>(lim);
 }
 
 /* Launch one FFT pass: the register kernel when the shape allows it, else the shared-memory
@@ -1920,24 +1979,7 @@ static void launch_fft_pass(const typename cplx<R>::T *in, typename cplx<R>::T *
           return;
         }
       }
-      if (L == 512) { /* the size-2^18 FFTs' two passes: a build for L = 512 */
-        if (tin && tout)
-          k_fft_reg<R, true, true, StridedLd<R>, false, 9><<<g, thr, sm, st>>>(sld, out, twM, twM, fmm_pass(fp),
-                                                                               nullptr, nullptr, O);
-        else if (tin)
-          k_fft_reg<R, true, false, StridedLd<R>, false, 9><<<g, thr, sm, st>>>(sld, out, twM, twM, fmm_pass(fp),
-                                                                                nullptr, nullptr, O);
-        else
-          k_fft_reg<R, false, false, StridedLd<R>, false, 9><<<g, thr, sm, st>>>(sld, out, twM, twM, fmm_pass(fp),
-                                                                                 nullptr, nullptr, O);
-        return;
-      }
-      if (tin && tout)
-        k_fft_reg<R, true, true><<<g, thr, sm, st>>>(sld, out, twM, twM, fmm_pass(fp), nullptr, nullptr, O);
-      else if (tin)
-        k_fft_reg<R, true, false><<<g, thr, sm, st>>>(sld, out, twM, twM, fmm_pass(fp), nullptr, nullptr, O);
-      else
-        k_fft_reg<R, false, false><<<g, thr, sm, st>>>(sld, out, twM, twM, fmm_pass(fp), nullptr, nullptr, O);
+      launch_fft_reg<R>(sld, out, twM, twM, fmm_pass(fp), tin, tout, g, thr, sm, st, O);
       return;
     }
   }
@@ -3304,12 +3346,11 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
       k_fft_reg<R, false, false, CombineLd<R>, true>
           <<<dim3((unsigned)(ccols / Wc), (unsigned)nbt), thr, sm + sizeof(C) * (size_t)(P + P / 16 + 1), st>>>(
               cl, cz, d->twP, d->twP, fp, d->twP_lo, d->twP_lo);
-    else if (P == 64) /* a build for 64 sections */
-      k_fft_reg<R, false, false, CombineLd<R>, false, 6><<<dim3((unsigned)(ccols / Wc), (unsigned)nbt), thr, sm, st>>>(
-          cl, cz, d->twP, d->twP, fp);
     else
-      k_fft_reg<R, false, false, CombineLd<R>><<<dim3((unsigned)(ccols / Wc), (unsigned)nbt), thr, sm, st>>>(
-          cl, cz, d->twP, d->twP, fp);
+      fft_by_len<kCombLo, kCombHi>((int)P, [&](auto lgt) { /* a build for each usual number of sections */
+        k_fft_reg<R, false, false, CombineLd<R>, false, decltype(lgt)::value>
+            <<<dim3((unsigned)(ccols / Wc), (unsigned)nbt), thr, sm, st>>>(cl, cz, d->twP, d->twP, fp);
+      });
   } else {
     pf.launches[ST_COMBINE]++;
     int TMc = (int)(P >= 1024 ? 1 : (1024 / P < 32 ? 1024 / P : 32));
@@ -3520,26 +3561,12 @@ static int set_smem_limits(void) {
   int lim = maxopt > 0 ? maxopt : 48 * 1024;
   cudaFuncSetAttribute(k_fft_pass<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_fft_pass<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute(k_fft_reg<float, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute(k_fft_reg<float, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute(k_fft_reg<float, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute(k_fft_reg<float, false, false, CombineLd<float>>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+  fft_smem_limit<float, 0, kFftHi>(lim);
+  fft_smem_limit<double, 0, kFftHi>(lim);
   cudaFuncSetAttribute(k_fft_reg<float, false, false, CombineLd<float>, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_fft_reg<float, true, true, StridedLd<float>, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_fft_reg<float, true, false, StridedLd<float>, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_fft_reg<float, false, false, StridedLd<float>, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute(k_fft_reg<double, false, false, CombineLd<double>>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute(k_fft_reg<double, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute(k_fft_reg<double, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute(k_fft_reg<double, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute(k_fft_reg<float, true, true, StridedLd<float>, false, 9>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute(k_fft_reg<float, true, false, StridedLd<float>, false, 9>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute(k_fft_reg<float, false, false, StridedLd<float>, false, 9>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute(k_fft_reg<double, true, true, StridedLd<double>, false, 9>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute(k_fft_reg<double, true, false, StridedLd<double>, false, 9>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute(k_fft_reg<double, false, false, StridedLd<double>, false, 9>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute(k_fft_reg<float, false, false, CombineLd<float>, false, 6>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute(k_fft_reg<double, false, false, CombineLd<double>, false, 6>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_combine<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_combine<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_sections<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
@@ -4498,12 +4525,7 @@ static int fft_run(fmmk_fft *f, const void *in, void *out, cudaStream_t st, char
     const size_t sm = sizeof(C) * fft_smem_elems(fp.L, fp.W);
     dim3 g((unsigned)(f->per[k] / fp.W), (unsigned)f->rows[k]);
     const StridedLd<R> sld{src, fp.irow, fp.iseq, (unsigned)fp.istr};
-    if (f->tin[k] && f->tout[k])
-      k_fft_reg<R, true, true><<<g, thr, sm, st>>>(sld, dst, twD, twP, fp);
-    else if (f->tin[k])
-      k_fft_reg<R, true, false><<<g, thr, sm, st>>>(sld, dst, twD, twP, fp);
-    else
-      k_fft_reg<R, false, false><<<g, thr, sm, st>>>(sld, dst, twD, twP, fp);
+    launch_fft_reg<R>(sld, dst, twD, twP, fp, f->tin[k], f->tout[k], g, thr, sm, st);
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
