@@ -20,7 +20,7 @@ NVCC = os.path.join(CUDA_HOME, "bin", "nvcc")
 
 CU_SOURCES = ["fmmfft_kernels.cu"]
 C_SOURCES = ["fmmfft_ops.c", "fmmfft_api.c", "fmmfft_serve.c"]
-HEADERS = ["fmmfft_internal.h", "fmmfft_tc.cuh", "fmmfft_tcss.cuh", "fmmfft_rows.cuh", "fmmfft_tree.cuh", "fmmfft_rows32.cuh",
+HEADERS = ["fmmfft_internal.h", "fmmfft_tc.cuh", "fmmfft_tcss.cuh", "fmmfft_rows.cuh", "fmmfft_tree.cuh", "fmmfft_rows32.cuh", "fmmfft_fftpair.cuh",
            os.path.join("..", "..", "include", "fmmfft.h")]
 
 NVCC_FLAGS = [

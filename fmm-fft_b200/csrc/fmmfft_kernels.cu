@@ -1902,6 +1902,8 @@ __global__ void __launch_bounds__(512, sizeof(R) == 4 ? 3 : 1)
   }
 }
 
+#include "fmmfft_fftpair.cuh"
+
 /* A build for each usual pass length, whose exchange addresses and stage loop are constants but for a few
  * XORs (2^26, P = 256: the combine 437 us in the build for any L, 357 in its own): f with log2 L as a
  * constant where it lies in LO .. HI, else 0 */
@@ -1929,9 +1931,39 @@ static void launch_fft_reg(const StridedLd<R> &ld, typename cplx<R>::T *out, con
       k_fft_reg<R, false, false, S, false, G><<<g, thr, sm, st>>>(ld, out, twD, twP, fp, nullptr, nullptr, O);
   });
 }
+/* Pairs of sequences a block of a paired FP32 pass (k_fft_pair), at most `most`; 0: the pass stays with
+ * k_fft_reg (a sequence by itself, blocks under a warp). */
+static int fft_pairs(int L, long per, int threads, int most) {
+  long np = threads / (L / 8);
+  if (np > most) np = most;
+  while (2 * np > per) np >>= 1;
+  return np * (L / 8) >= 32 ? (int)np : 0;
+}
+static void launch_fft_pair(const StridedLd<float> &ld, float2 *out, const float2 *twD, const float2 *twP, FftPass fp, bool tin,
+                            bool tout, int np, long per, long rows, cudaStream_t st, const OutTab &O = OutTab{}) {
+  fp.W = 2 * np;
+  const dim3 g((unsigned)(per / fp.W), (unsigned)rows);
+  const int thr = np * (fp.L / 8);
+  const size_t sm = pair_smem(fp.L, np);
+  const StridedLd2 ld2{ld};
+  fft_by_len<kFftLo, kFftHi>(fp.L, [&](auto lgt) {
+    constexpr int G = decltype(lgt)::value;
+    if (tin && tout) k_fft_pair<true, true, StridedLd2, G><<<g, thr, sm, st>>>(ld2, out, twD, twP, fp, O);
+    else if (tin) k_fft_pair<true, false, StridedLd2, G><<<g, thr, sm, st>>>(ld2, out, twD, twP, fp, O);
+    else k_fft_pair<false, false, StridedLd2, G><<<g, thr, sm, st>>>(ld2, out, twD, twP, fp, O);
+  });
+}
 /* the shared-memory opt-in of every build */
 template <typename R, int G, int HI> static void fft_smem_limit(int lim) {
   constexpr auto at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  if constexpr (sizeof(R) == 4) {
+    if constexpr (G == 0 || (G >= kFftLo && G <= kFftHi)) {
+      cudaFuncSetAttribute(k_fft_pair<true, true, StridedLd2, G>, at, lim);
+      cudaFuncSetAttribute(k_fft_pair<true, false, StridedLd2, G>, at, lim);
+      cudaFuncSetAttribute(k_fft_pair<false, false, StridedLd2, G>, at, lim);
+    }
+    if constexpr (G == 0 || (G >= kCombLo && G <= kCombHi)) cudaFuncSetAttribute(k_fft_pair<false, false, CombineLd2, G>, at, lim);
+  }
   if constexpr (G == 0 || (G >= kFftLo && G <= kFftHi)) {
     cudaFuncSetAttribute(k_fft_reg<R, true, true, StridedLd<R>, false, G>, at, lim);
     cudaFuncSetAttribute(k_fft_reg<R, true, false, StridedLd<R>, false, G>, at, lim);
@@ -1953,6 +1985,13 @@ static void launch_fft_pass(const typename cplx<R>::T *in, typename cplx<R>::T *
   const OutTab O = ot ? *ot : OutTab{}; /* the last pass of a pointer-table execute */
   const int L = fp.L;
   const bool tin = fp.istr == 1, tout = fp.ostr == 1;
+  if constexpr (sizeof(R) == 4) {
+    const int np = L >= 16 && L <= 8 * reg_threads && !(tout && !tin) && !twM_lo ? fft_pairs(L, per, reg_threads, 8) : 0;
+    if (np >= (tin ? 1 : 2)) {
+      launch_fft_pair({in, fp.M, fp.iseq, (unsigned)fp.istr}, out, twM, twM, fmm_pass(fp), tin, tout, np, per, rows, st, O);
+      return;
+    }
+  }
   if (L >= 16 && L <= 8 * reg_threads && !(tout && !tin)) {
     int W = reg_threads / (L / 8);
     if (W > 16) W = 16;
@@ -3346,7 +3385,17 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
       k_fft_reg<R, false, false, CombineLd<R>, true>
           <<<dim3((unsigned)(ccols / Wc), (unsigned)nbt), thr, sm + sizeof(C) * (size_t)(P + P / 16 + 1), st>>>(
               cl, cz, d->twP, d->twP, fp, d->twP_lo, d->twP_lo);
-    else
+    else if (const int np = sizeof(R) == 4 ? fft_pairs((int)P, ccols, 512, 32) : 0) {
+      if constexpr (sizeof(R) == 4) {
+        fp.W = 2 * np;
+        const CombineLd2 cl2{cl};
+        fft_by_len<kCombLo, kCombHi>((int)P, [&](auto lgt) {
+          k_fft_pair<false, false, CombineLd2, decltype(lgt)::value>
+              <<<dim3((unsigned)(ccols / fp.W), (unsigned)nbt), np * (int)(P / 8), pair_smem((int)P, np), st>>>(
+                  cl2, cz, d->twP, d->twP, fp, OutTab{});
+        });
+      }
+    } else
       fft_by_len<kCombLo, kCombHi>((int)P, [&](auto lgt) { /* a build for each usual number of sections */
         k_fft_reg<R, false, false, CombineLd<R>, false, decltype(lgt)::value>
             <<<dim3((unsigned)(ccols / Wc), (unsigned)nbt), thr, sm, st>>>(cl, cz, d->twP, d->twP, fp);
@@ -4525,6 +4574,13 @@ static int fft_run(fmmk_fft *f, const void *in, void *out, cudaStream_t st, char
     const size_t sm = sizeof(C) * fft_smem_elems(fp.L, fp.W);
     dim3 g((unsigned)(f->per[k] / fp.W), (unsigned)f->rows[k]);
     const StridedLd<R> sld{src, fp.irow, fp.iseq, (unsigned)fp.istr};
+    if constexpr (sizeof(R) == 4) {
+      const int np = fft_pairs(fp.L, f->per[k], 512, 8);
+      if (np >= (f->tin[k] ? 1 : 2)) {
+        launch_fft_pair(sld, dst, twD, twP, fp, f->tin[k], f->tout[k], np, f->per[k], f->rows[k], st);
+        continue;
+      }
+    }
     launch_fft_reg<R>(sld, dst, twD, twP, fp, f->tin[k], f->tout[k], g, thr, sm, st);
   }
   cudaError_t e = cudaGetLastError();
