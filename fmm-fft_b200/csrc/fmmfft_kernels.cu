@@ -193,7 +193,6 @@ template <typename R> struct Dev {
   unsigned *sync;   /* grid barrier of the coarse-tree kernel: [0] arrivals, [32] generation */
   long coarse_rows; /* levels with fewer rows go to the coarse-tree kernel (0: none) */
   int coarse_grid;  /* blocks of the coarse-tree kernel an SM holds (0: its operators do not fit) */
-  int coarse_dbuf;  /* the coarse-tree kernel's operators in two alternating buffers */
   int fuse_s2m;     /* S2M inside the sections pass where tiles hold whole boxes */
   /* FP64 plans: tree stages and leaf as row contractions on the FP64 matrix instructions
    * (fmmfft_rows.cuh) and their operators */
@@ -2109,215 +2108,6 @@ __global__ void k_block_dc(const typename cplx<R>::T *__restrict__ ssum,
   }
 }
 
-/* ======================================================================== coarse tree */
-
-/* The coarse levels of the tree (few boxes: every level whose row count per transform is below
- * a threshold, at most 2^kCoarseMaxLevel boxes per plane) in one launch instead of one launch per
- * level: the upward M2M for parent levels Lm .. 2, the top flip, and the downward M2L + L2L for
- * child levels 3 .. Ll.  Every expansion plane (section, re/im, transform) is independent of the
- * others at every level (its neighbours wrap within the plane), so one block takes one plane
- * through all of these levels.  The plane's coarse levels stay in shared memory: phi of the
- * levels above Lm (made by the per-level kernels) is read from global memory once, every level
- * computed here is kept in shared memory for the levels after it and written to global memory
- * once (the per-level kernels after this one and the debug views read it there), so a level
- * costs one block barrier and no global round trip.  The levels' operators are copied with
- * cp.async into two alternating buffers, the next level's while the current one computes (one
- * buffer, copied after the barrier, when two do not fit).  Same operators, layouts and outputs
- * as the per-level launches (reference fmmfft.c:476-515 upward, :620-749 top and downward).
- * Compute: one warp per output row, lane = output column (N / 32 columns per lane); the K sum
- * accumulates per 32-column block, then into the total (two-level FP32 accumulation, as in the
- * row kernels).  Launched as a programmatic dependent launch: the first operator is staged
- * before the wait for the kernel that made its input. */
-template <typename R> struct CoarseArgs {
-  R *phi, *psi;
-  const R *bm2m, *btop, *bm2l;
-  long S1; /* planes / 2, all transforms of the execute */
-  int T, Lm, Ll; /* coarse M2M parent levels Lm..2 (none when Lm < 2); M2L child levels 3..Ll */
-  int dbuf;      /* two operator buffers */
-};
-constexpr int kCoarseMaxLevel = 6; /* coarse M2M parents hold at most 2^6 boxes per plane */
-constexpr int kCoarseWarps = 32;   /* a block: one warp per row */
-constexpr int kCoarseTop = kCoarseMaxLevel + 1; /* highest level a block holds (M2M input, M2L) */
-
-__device__ __forceinline__ void cp_async_wait0() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-
-/* Issue the copy of a level's operator B (K x N, row-major) into the shared array Bs with
- * cp.async, in 16-byte pieces where the size and address allow, else one element per copy;
- * nothing waits here. */
-template <typename R>
-__device__ __forceinline__ void coarse_stage_b(int K, int N, const R *__restrict__ B, R *__restrict__ Bs) {
-  const int n = K * N;
-  const uint32_t sb = (uint32_t)__cvta_generic_to_shared(Bs);
-  if (((size_t)n * sizeof(R)) % 16 == 0 && ((uintptr_t)B & 15) == 0 && (sb & 15) == 0) {
-    constexpr int per = 16 / sizeof(R);
-    for (int e = threadIdx.x * per; e < n; e += blockDim.x * per)
-      tc::cp_async16(sb + (uint32_t)(e * sizeof(R)), B + e);
-  } else {
-    for (int e = threadIdx.x; e < n; e += blockDim.x) {
-      if constexpr (sizeof(R) == 8)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" : : "r"(sb + (uint32_t)(e * 8)), "l"(B + e) : "memory");
-      else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" : : "r"(sb + (uint32_t)(e * 4)), "l"(B + e) : "memory");
-    }
-  }
-  asm volatile("cp.async.commit_group;" ::: "memory");
-}
-
-/* Floats (elements) of a plane's levels 2..L: (2^(L+1) - 4) rows of T. */
-__host__ __device__ constexpr long coarse_lvl_rows(int L) { return (2L << L) - 4; }
-
-/* Shared memory of the coarse kernel: one or two operator buffers (the largest operator, the
- * M2L one, 5T x 2T), the plane's phi and psi levels 2..kCoarseTop and the split-K partial sums
- * (at most 32 rows x parts of 2T). */
-template <typename R> static size_t coarse_smem(long T, int dbuf) {
-  return sizeof(R) * ((dbuf ? 20 : 10) * (size_t)T * T + 2 * (size_t)coarse_lvl_rows(kCoarseTop) * T +
-                      (size_t)kCoarseWarps * 4 * T);
-}
-
-/* Rows [0, rows) of one level: out[r][n] = sum_k A(r, k) Bs[k][n].  Row r's A is up to three
- * contiguous pieces of shared memory, segs(r, p, o) filling piece pointers p[] and their first K
- * index o[] (o[0] = 0, pieces in K order, o[3] = K).  A level with fewer rows than warps splits
- * each row's K range over S = warps / rows warps (S <= 8); their partial sums go to `red` and are
- * added in a fixed order (so a plane's bits do not depend on anything else).  Lane = output
- * column (NJ columns per lane, N <= 32 NJ).  Outputs go to the shared level Os and to global
- * memory Og.  Ends with the outputs written by the threads that wrote them (the caller's next
- * barrier publishes them). */
-template <typename R, int NJ, class Segs>
-__device__ __forceinline__ void coarse_level(int rows, int K, int N, const R *__restrict__ Bs, R *__restrict__ Os,
-                                             R *__restrict__ Og, R *__restrict__ red, Segs segs) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int S = kCoarseWarps / rows;
-  S = S < 1 ? 1 : (S > 8 ? 8 : S);
-  const int kper = (K + S - 1) / S;
-  for (int it = warp; it < rows * S; it += kCoarseWarps) {
-    const int r = it / S, part = it - r * S;
-    const int k0 = part * kper, k1 = k0 + kper < K ? k0 + kper : K;
-    const R *pc[3];
-    int o[4];
-    segs(r, pc, o);
-    R acc[NJ];
-#pragma unroll
-    for (int j = 0; j < NJ; ++j) acc[j] = R(0);
-    for (int q = 0; q < 3; ++q) {
-      const int lo = k0 > o[q] ? k0 : o[q], hi = k1 < o[q + 1] ? k1 : o[q + 1];
-      const R *ap = pc[q];
-#pragma unroll 4
-      for (int k = lo; k < hi; ++k) {
-        const R av = ap[k - o[q]];
-        const R *bk = Bs + k * N + lane;
-#pragma unroll
-        for (int j = 0; j < NJ; ++j)
-          if (NJ == 1 || lane + 32 * j < N) acc[j] = fma(av, bk[32 * j], acc[j]);
-      }
-    }
-    if (S == 1) {
-#pragma unroll
-      for (int j = 0; j < NJ; ++j)
-        if (lane + 32 * j < N) Os[r * N + lane + 32 * j] = acc[j], Og[r * N + lane + 32 * j] = acc[j];
-    } else {
-#pragma unroll
-      for (int j = 0; j < NJ; ++j)
-        if (lane + 32 * j < N) red[it * N + lane + 32 * j] = acc[j];
-    }
-  }
-  if (S > 1) {
-    __syncthreads();
-    for (int e = threadIdx.x; e < rows * N; e += blockDim.x) {
-      const int r = e / N, c = e - r * N;
-      R v = red[(r * S) * N + c];
-      for (int part = 1; part < S; ++part) v += red[(r * S + part) * N + c];
-      Os[e] = v;
-      Og[e] = v;
-    }
-  }
-}
-
-/* the same with the lane's column count chosen from N */
-template <typename R, class Segs>
-__device__ __forceinline__ void coarse_level_n(int rows, int K, int N, const R *Bs, R *Os, R *Og, R *red, Segs segs) {
-  if (N <= 32) coarse_level<R, 1>(rows, K, N, Bs, Os, Og, red, segs);
-  else if (N <= 64) coarse_level<R, 2>(rows, K, N, Bs, Os, Og, red, segs);
-  else coarse_level<R, 4>(rows, K, N, Bs, Os, Og, red, segs);
-}
-
-template <typename R> __global__ void __launch_bounds__(32 * kCoarseWarps) k_coarse(CoarseArgs<R> a) {
-  extern __shared__ __align__(16) unsigned char coarse_raw[];
-  const int T = a.T;
-  R *Bs[2];
-  Bs[0] = reinterpret_cast<R *>(coarse_raw);
-  Bs[1] = a.dbuf ? Bs[0] + 10L * T * T : Bs[0];
-  R *Ph = Bs[0] + (a.dbuf ? 20L : 10L) * T * T; /* phi levels 2..kCoarseTop of this plane */
-  R *Ps = Ph + coarse_lvl_rows(kCoarseTop) * T; /* psi levels 2..kCoarseTop */
-  R *red = Ps + coarse_lvl_rows(kCoarseTop) * T; /* split-K partial sums: 32 x 4T */
-  const long S1 = a.S1, pl = blockIdx.x;
-  /* level l of this block's plane, in global and in shared memory */
-  auto lv = [&](R *base, int l) { return base + lvl_off(l, S1, T) + pl * (1L << l) * T; };
-  auto sl = [&](R *base, int l) { return base + ((1L << l) - 4) * T; };
-  /* the levels in order: M2M parents Lm..2, the top flip, M2L children 3..Ll */
-  const int nm = a.Lm >= 2 ? a.Lm - 1 : 0, nlev = nm + 1 + (a.Ll >= 3 ? a.Ll - 2 : 0);
-  auto stage_op = [&](int i, R *dst) {
-    if (i < nm) coarse_stage_b<R>(2 * T, T, a.bm2m + (long)(a.Lm - i - 2) * 2 * T * T, dst);
-    else if (i == nm) coarse_stage_b<R>(T, T, a.btop, dst);
-    else coarse_stage_b<R>(5 * T, 2 * T, a.bm2l + (long)(i - nm - 1) * 10 * T * T, dst);
-  };
-  tc::pdl_trigger();
-  stage_op(0, Bs[0]); /* a plan constant */
-  tc::pdl_wait();
-  { /* phi of the levels this block does not make: Lm+1 .. Ltop (only Lm+1 when the M2M runs
-     * here; the top flip and M2L read levels 2..Ll) */
-    const int lo = a.Lm >= 2 ? a.Lm + 1 : 2;
-    const int hi = a.Ll > lo ? a.Ll : lo;
-    for (int l = lo; l <= hi; ++l) {
-      const R *g = lv(a.phi, l);
-      R *d = sl(Ph, l);
-      const int n = (1 << l) * T;
-      for (int e = threadIdx.x; e < n; e += blockDim.x) d[e] = g[e];
-    }
-  }
-  for (int i = 0; i < nlev; ++i) {
-    R *B = Bs[i & 1];
-    if (a.dbuf) {
-      cp_async_wait0(); /* this thread's copies of level i's operator */
-      __syncthreads();  /* everyone's; the level before is written and done with the other buffer */
-      if (i + 1 < nlev) stage_op(i + 1, Bs[(i + 1) & 1]);
-    } else {
-      if (i > 0) {
-        __syncthreads(); /* the level before is done with the buffer */
-        stage_op(i, B);
-      }
-      cp_async_wait0();
-      __syncthreads();
-    }
-    if (i < nm) { /* M2M: parent level L from child pairs of L + 1 */
-      const int L = a.Lm - i;
-      const R *child = sl(Ph, L + 1);
-      coarse_level_n<R>(1 << L, 2 * T, T, B, sl(Ph, L), lv(a.phi, L), red, [=](int r, const R **p, int *o) {
-        p[0] = child + r * 2 * T, p[1] = p[2] = p[0];
-        o[0] = 0, o[1] = o[2] = o[3] = 2 * T;
-      });
-    } else if (i == nm) { /* top flip: psi_2[c] = topflp . phi_2[(c + 2) mod 4] */
-      const R *phi2 = sl(Ph, 2);
-      coarse_level_n<R>(4, T, T, B, sl(Ps, 2), lv(a.psi, 2), red, [=](int r, const R **p, int *o) {
-        p[0] = phi2 + ((r + 2) & 3) * T, p[1] = p[2] = p[0];
-        o[0] = 0, o[1] = o[2] = o[3] = T;
-      });
-    } else { /* M2L + L2L: child level l, one row per parent box: psi of the parent, then the
-              * child pairs 2r-2, 2r-1 and 2r+2, 2r+3 (wrapping; a pair never straddles the end) */
-      const int l = i - nm + 2;
-      const R *psi_par = sl(Ps, l - 1), *phi = sl(Ph, l);
-      const int mask = (1 << l) - 1;
-      coarse_level_n<R>(1 << (l - 1), 5 * T, 2 * T, B, sl(Ps, l), lv(a.psi, l), red,
-                        [=](int r, const R **p, int *o) {
-                          p[0] = psi_par + r * T;
-                          p[1] = phi + ((2 * r - 2) & mask) * T;
-                          p[2] = phi + ((2 * r + 2) & mask) * T;
-                          o[0] = 0, o[1] = T, o[2] = 3 * T, o[3] = 5 * T;
-                        });
-    }
-  }
-  cp_async_wait0();
-}
-
 /* Self-test of the bounded device waits: the same wait routine as the tensor-core kernels
  * (tc::t_wait on an mbarrier, with tensor memory held), made to wait for an event that never
  * comes (an mbarrier nobody arrives on) with a short limit.  The wait gives up, records the error
@@ -2595,15 +2385,15 @@ constexpr long kCoarseRows = 4096; /* default: tree levels with fewer rows form 
 template <typename R> static void coarse_setup(Dev<R> *d) {
   d->coarse_rows = kCoarseRows;
   if (const char *ev = getenv("FMMFFT_COARSE_ROWS")) d->coarse_rows = atol(ev), d->env_set |= KNOB_COARSE;
-  /* two operator buffers where they fit beside the plane's levels, else one */
-  d->coarse_dbuf = coarse_smem<R>(d->T, 1) <= (size_t)200 * 1024;
-  const size_t sm = coarse_smem<R>(d->T, d->coarse_dbuf);
+  /* one operator at a time beside the most levels a block may hold */
+  using E = typename TreeEng<R>::E;
+  const size_t sm = coarse_smem<E>((int)d->T, kCoarseMaxLevel, kCoarseMaxLevel + 1, 0);
   int nb = 0;
   if (sm <= (size_t)200 * 1024) {
     /* the attribute is the kernel's, not the plan's: always the full allowance, so that a plan
      * with fewer terms made later does not shrink what an earlier plan's launch needs */
-    cudaFuncSetAttribute(k_coarse<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_coarse<R>, 32 * kCoarseWarps, sm);
+    cudaFuncSetAttribute(k_coarse<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_coarse<E>, kCoarseThreads, sm);
   }
   d->coarse_grid = nb;
   if (d->coarse_grid < 1) d->coarse_rows = 0; /* operator too large for shared memory */
@@ -2740,9 +2530,11 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
   if (!shard) tree_setup<R>(d); /* a shard runs its stages in pieces */
   if (d->tree) d->ok_s2m = d->ok_m2m = d->ok_m2l = d->ok_leaf = d->ok_lnb = 0; /* no stage reaches them */
   /* a small level's row contraction costs 3 to 4 us, less than the same level in the coarse tree from
-   * about 1024 rows (N = 2^20, P = 32, 15 terms, levels from 4096 / 1024 / 256 rows: 150 / 140 / 140 us a
-   * transform; N = 2^17, 24 terms: 96 / 74 / 75) */
-  if (d->rows && d->coarse_rows > kRowsMinRows) d->coarse_rows = kRowsMinRows;
+   * about 1024 rows in FP64 and 2048 in FP32 (levels from 1024 / 2048 / 4096 rows, us a transform: FP64 2^20, P =
+   * 32, 15 terms 145 / 148 / 146; FP32 2^20, P = 64, 20 terms 123 / 121 / 123; split TF32 2^24, 24 terms 816 / 819 /
+   * 827; 2^22, P = 256, 16 terms 239 / 236 / 233) */
+  const long rows_min = sizeof(R) == 8 ? kRowsMinRows : 2 * kRowsMinRows;
+  if (d->rows && d->coarse_rows > rows_min) d->coarse_rows = rows_min;
   const long sz_s2m = d->ok_s2m ? (long)d->kp_s2m * d->np_s2m : 0;
   d->tc_s2m_stride16 = 2L * tc::round16(d->kp_s2m) * d->np_s2m;
   d->tc_m2m_stride16 = 2L * tc::round16(d->kp_m2m) * d->np_m2m;
@@ -2808,7 +2600,8 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
   CARVE(wsm2l, ws_m2l_n, float)
   CARVE(wsleaf, ws_leaf_n, float)
   CARVE(tstages, d->tree ? 2 * kTreeStages : 0, TreeStage)
-  CARVE(tops, d->rows || d->tree ? tree_nops<E>(P, T, b, nlev) : 0, R)
+  const long ntops = tree_nops<E>(d->rows || d->tree ? P : 1, T, b, nlev); /* the leaf's for row contractions only */
+  CARVE(tops, ntops, R)
 #undef CARVE
   if (dry_bytes) {
     *dry_bytes = off;
@@ -2940,7 +2733,7 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
   free(hm);
   if (tc && !rc) rc = tc_upload_ops(d, o, err, errlen);
   if (d->ss_leaf && !rc) ss_smem_limits();
-  if ((d->rows || d->tree) && !rc) {
+  if (!rc) {
     if (d->rows) sizeof(R) == 8 ? rows_smem_limits((int)T, (int)b) : rows32_smem_limits();
     if (d->tree) {
       TreeStage hs[2 * kTreeStages];
@@ -2948,7 +2741,7 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
       if (cudaMemcpy(d->tstages, hs, sizeof hs, cudaMemcpyHostToDevice) != cudaSuccess) rc = 3;
     }
     k_tree_ops<E><<<2 * d->num_sms, 256>>>(d->tops, d->initch, d->bm2m, d->bm2l, d->btop, d->evalmT, d->cot,
-                                           tree_nops<E>(P, T, b, nlev), (int)T, (int)b, (int)nlev);
+                                           ntops, (int)T, (int)b, (int)nlev);
     if (cudaStreamSynchronize(0) != cudaSuccess) { /* the plan's executes may run on any stream */
       snprintf(err, errlen, "operator layout: %s", cudaGetErrorString(cudaGetLastError()));
       rc = 3;
@@ -3179,20 +2972,24 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
   stage(ST_TOP);
   if (!run(ST_TOP)) {
   } else if (coarse) {
-    CoarseArgs<R> ca{d->phi, d->psi, d->bm2m, d->btop, d->bm2l, S1e, (int)T, (int)Lm, (int)Ll, d->coarse_dbuf};
+    using E = typename TreeEng<R>::E;
+    CoarseArgs<E> ca{d->phi, d->psi, rop.m2m, rop.m2l, rop.top, S1e, (int)T, (int)Lm, (int)Ll};
+    /* every operator at once where two blocks an SM still fit */
+    ca.resident = coarse_smem<E>((int)T, (int)Lm, (int)Ll, 1) <= (size_t)110 * 1024;
+    coarse_stages<E>(ca);
     /* one block per expansion plane of every transform of the execute; a programmatic dependent
-     * launch (it stages its first operator before waiting for the level below) */
+     * launch (it stages its operators before waiting for the level below) */
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(2 * S1e));
-    cfg.blockDim = dim3(32 * kCoarseWarps);
-    cfg.dynamicSmemBytes = coarse_smem<R>(T, d->coarse_dbuf);
+    cfg.blockDim = dim3(kCoarseThreads);
+    cfg.dynamicSmemBytes = coarse_smem<E>((int)T, (int)Lm, (int)Ll, ca.resident);
     cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = d->pdl ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, k_coarse<R>, ca);
+    cudaLaunchKernelEx(&cfg, k_coarse<E>, ca);
     pf.launches[ST_TOP]++;
   } else {
     ProbTop<R> pb{d->phi + lvl_off(2, S1e, T), d->btop, d->psi + lvl_off(2, S1e, T), 2 * S1e * 4,

@@ -4,8 +4,7 @@
  *
  * Every section of the transform is a tree of its own from its samples to its field, so sections of
  * up to a few thousand points need no launch between levels, no planar copy of the samples and no
- * pass for their sums; and the one-block-per-plane coarse tree, which had most of such a transform's
- * time, computes a level with one warp per row, two shared loads an FMA.  Here a stage costs two
+ * pass for their sums.  Here a stage costs two
  * block barriers, and its contraction is blk_gemm: out[row][c] = sum_k A(row, k) B[k][c], A rows and B
  * in shared memory, a thread (FP32) a register tile of the output, a warp (FP64) tiles of the FP64
  * matrix instruction.  Bound by latency: a stage of a small section is a chain of a few hundred
@@ -74,7 +73,7 @@ __global__ void k_tree_ops(typename E::R *__restrict__ out, const typename E::R 
     R v = 0;
     if (e < n_s2m) {
       E::kc(e, Tn, k, c);
-      if (c < T) v = initch[k * T + c];
+      if (k < b && c < T) v = initch[k * T + c];
     } else if (e < n_top) {
       const long q = e < n_m2m ? e - n_s2m : e < n_m2l ? e - n_m2m : e - n_m2l, g = q / blk;
       E::kc(q - g * blk, Tn, k, c);
@@ -489,6 +488,121 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 5 : 1) k_tree(const __grid_con
       const int row = r * npar + par;
       if (so >= 0) tree_sput2<R>(sm + so + row * Tq + c, v0, v1);
       else if (c == 0 && shifted) v0 = 2 * sc == a.P ? R(0.5) * (v0 + sm[lay.hv + row]) : sm[lay.hv + row];
+      tree_put2<R>(gbase + (long)row * gn, gn, c, v0, v1);
+    });
+  }
+}
+
+/* ------------------------------------------------------------------------ the coarse levels of a large tree */
+/* The levels of few boxes in one launch, a block an expansion plane (section, re/im, transform; planes are
+ * independent at every level): M2M for parent levels Lm .. 2, the top flip, M2L + L2L for child levels
+ * 3 .. Ll, each a stage of blk_gemm between two barriers.  phi of the level below comes from global
+ * memory, every level made here goes there too (the row contractions and the debug views read it).  A
+ * launch a level costs 3 to 4 us.  Bound by latency, like k_tree: us a launch, with one warp an output row
+ * and two shared loads an FMA -> this: FP32 2^20, P = 64, 20 terms 18.4 -> 14.1; FP64 2^20, P = 32, 15 terms
+ * 22.6 -> 14.4; FP64 2^17, P = 16, 24 terms 49 -> 29 (512 threads a block: the same, and 14 -> 23 at P = 256). */
+constexpr int kCoarseMaxLevel = 6; /* M2M parents hold at most 2^6 boxes a plane */
+constexpr int kCoarseStages = 2 * (kCoarseMaxLevel - 1) + 1, kCoarseThreads = 256;
+
+template <class E> struct CoarseArgs {
+  using R = typename E::R;
+  R *phi, *psi;
+  const R *m2m, *m2l, *top; /* TreeOps */
+  long S1;                  /* planes / 2, all transforms of the execute */
+  int T, Lm, Ll, resident, ns;
+  TreeStage st[kCoarseStages];
+};
+/* Shared layout, in values: operators (all, or a buffer for one), phi levels 2 .. top, two levels of psi; the
+ * stage table follows. */
+template <class E> struct CoarseLay {
+  int top, ph, ps[2], end;
+  __host__ __device__ CoarseLay(int T, int Lm, int Ll, int resident) {
+    const int Tq = tree_pitch(rows_kpad(T)), blk = tree_blk<E>(T);
+    top = Lm >= 2 ? Lm + 1 : 2;
+    if (Ll > top) top = Ll;
+    ph = (resident ? 2 * (Lm - 1) + 1 + 8 * (Ll - 2) : Ll >= 3 ? 8 : 2) * blk;
+    ps[0] = ph + ((2 << top) - 4) * Tq, ps[1] = ps[0] + (1 << Ll) * Tq, end = ps[1] + (Ll > 3 ? 1 << (Ll - 1) : 4) * Tq;
+  }
+};
+template <class E> static size_t coarse_smem(int T, int Lm, int Ll, int resident) {
+  return sizeof(typename E::R) * (size_t)CoarseLay<E>(T, Lm, Ll, resident).end + sizeof(TreeStage) * kCoarseStages;
+}
+template <class E> static void coarse_stages(CoarseArgs<E> &a) {
+  const int T = a.T, Tp = rows_kpad(T), Tq = tree_pitch(Tp), blk = tree_blk<E>(T), nm = a.Lm - 1;
+  const CoarseLay<E> lay(T, a.Lm, a.Ll, a.resident);
+  auto phl = [&](int l) { return lay.ph + ((1 << l) - 4) * Tq; };
+  auto psl = [&](int l) { return lay.ps[(a.Ll - l) & 1]; };
+  a.ns = nm + 1 + a.Ll - 2;
+  for (int i = 0; i < a.ns; ++i) {
+    TreeStage g{};
+    const int lM = a.Lm - i, lL = i - nm + 2; /* level of an M2M, of an M2L stage */
+    g.op = !a.resident ? 0 : i < nm ? (lM - 2) * 2 * blk : i == nm ? nm * 2 * blk : (nm * 2 + 1 + (lL - 3) * 8) * blk;
+    auto seg = [&](int base, int csh, int mul, int d0, int d1, int b0, int b1) {
+      g.seg[g.nseg++] = TreeSeg{base, Tq, csh, mul, {d0, d1}, Tp, {g.op + b0 * blk, g.op + b1 * blk}};
+    };
+    g.npar = 1, g.ncol = Tp, g.gn = T, g.lv = 2;
+    if (i < nm) {
+      g.lv = lM, g.rows = 1 << lM, g.rsh = lM, g.so = phl(lM), g.nop = 2 * blk;
+      seg(phl(lM + 1), lM + 1, 2, 0, 0, 0, 0), seg(phl(lM + 1), lM + 1, 2, 1, 1, 1, 1);
+    } else if (i == nm) {
+      g.rows = 4, g.rsh = 2, g.so = psl(2), g.nop = blk;
+      seg(phl(2), 2, 1, 2, 2, 0, 0);
+    } else {
+      g.lv = lL, g.rows = 1 << (lL - 1), g.rsh = lL - 1, g.npar = 2, g.so = psl(lL), g.nop = 8 * blk;
+      seg(psl(lL - 1), lL - 1, 1, 0, 0, 0, 4);
+      seg(phl(lL), lL, 2, -2, -3, 1, 5), seg(phl(lL), lL, 2, 2, -2, 2, 6), seg(phl(lL), lL, 2, 3, 2, 3, 7);
+    }
+    const unsigned ncx = (unsigned)((sizeof(typename E::R) == 8 ? (g.ncol + 7) / 8 : (g.ncol + 3) / 4) * g.npar);
+    g.rcp = ncx == 1 ? 0u : (unsigned)((0x100000000ull + ncx - 1) / ncx);
+    a.st[i] = g;
+  }
+}
+
+template <class E> __global__ void __launch_bounds__(kCoarseThreads) k_coarse(const __grid_constant__ CoarseArgs<E> a) {
+  using R = typename E::R;
+  extern __shared__ __align__(16) unsigned char tree_raw[];
+  R *const sm = reinterpret_cast<R *>(tree_raw);
+  const int T = a.T, Tp = rows_kpad(T), Tq = tree_pitch(Tp), blk = tree_blk<E>(T), nm = a.Lm - 1, ns = a.ns;
+  const CoarseLay<E> lay(T, a.Lm, a.Ll, a.resident);
+  TreeStage *const stages = reinterpret_cast<TreeStage *>(sm + lay.end);
+  const long pl = blockIdx.x;
+  auto stage_op = [&](int i) {
+    const R *src = i < nm ? a.m2m + (long)(a.Lm - i - 2) * 2 * blk : i == nm ? a.top : a.m2l + (long)(i - nm - 1) * 8 * blk;
+    tree_stage<R>(sm, src, a.st[i].nop);
+  };
+  tc::pdl_trigger();
+  /* plan constants, before the wait for the kernel that made phi */
+  if (a.resident) {
+    tree_stage<R>(sm, a.m2m, nm * 2 * blk);
+    tree_stage<R>(sm + nm * 2 * blk, a.top, blk);
+    tree_stage<R>(sm + (nm * 2 + 1) * blk, a.m2l, (a.Ll - 2) * 8 * blk);
+  } else {
+    stage_op(0);
+  }
+  tree_commit();
+  for (int e = threadIdx.x; e < ns * (int)(sizeof(TreeStage) / 4); e += kCoarseThreads)
+    reinterpret_cast<int *>(stages)[e] = reinterpret_cast<const int *>(a.st)[e];
+  tc::pdl_wait();
+  for (int l = a.Lm >= 2 ? a.Lm + 1 : 2; l <= lay.top; ++l) { /* phi of the levels not made here */
+    const R *src = a.phi + lvl_off(l, a.S1, T) + pl * (1L << l) * T;
+    R *const dst = sm + lay.ph + ((1 << l) - 4) * Tq;
+    for (int r = threadIdx.x >> 3; r < 1 << l; r += kCoarseThreads / 8)
+      for (int c = threadIdx.x & 7; c < Tp; c += 8) dst[r * Tq + c] = c < T ? src[r * T + c] : R(0);
+  }
+  for (int i = 0; i < ns; ++i) {
+    if (!a.resident && i > 0) {
+      __syncthreads(); /* the stage before is done with the operator buffer */
+      stage_op(i);
+      tree_commit();
+    }
+    if (i == 0 || !a.resident) tree_wait<0>();
+    __syncthreads(); /* this stage's operator and the stage before are in place */
+    const TreeStage &sg = stages[i];
+    R *const gbase = (i < nm ? a.phi : a.psi) + lvl_off(sg.lv, a.S1, T) + pl * (1L << sg.lv) * T;
+    const int so = sg.so, gn = sg.gn, npar = sg.npar;
+    blk_gemm(sm, sg, kCoarseThreads, [&](int r, int par, int c, R v0, R v1) {
+      const int row = r * npar + par;
+      tree_sput2<R>(sm + so + row * Tq + c, v0, v1);
       tree_put2<R>(gbase + (long)row * gn, gn, c, v0, v1);
     });
   }
