@@ -12,21 +12,26 @@
  *   4  M2M             row contraction per level: phi_L = [phi_L+1 pair] . [S_L;S_R]  (:476-515)
  *   5  top flip        psi_2[c] = topflp . phi_2[c+2]                    (:620-639)
  *   6  M2L + L2L       row contraction per level over parent boxes, both children at once
- *                      (:643-749); the tree levels of stages 4-6 with fewer than 4096 rows (at
- *                      most 64 boxes per plane) run in one launch, k_coarse, a block per plane
+ *                      (:643-749); the tree levels of stages 4-6 with few rows (FP64 under
+ *                      1024, FP32 under 2048; at most 64 boxes per plane) run in one launch,
+ *                      k_coarse, a block per plane
  *   7  leaf            row contraction per section: u = [psi_n | x window] . [E_sc ; cot
  *                      Toeplitz] with the half-shifted first point as one more operator column
- *                      (tensor cores) + k_leaf_mid for section P/2; k_leaf (direct, CUDA cores)
- *                      for FP32 / FP64 plans; rowgemm + k_leaf_fix when b % 8 != 0 (:751-954)
+ *                      (tensor cores) + k_leaf_mid for section P/2; row contractions for FP32 /
+ *                      FP64 plans (k_leaf, direct, for shapes they do not take); rowgemm +
+ *                      k_leaf_fix when b % 8 != 0 (:751-954)
  *   8  combine         pre-twiddle and length-P DFT over sections, transposed store, as a
- *                      register Stockham pass (k_fft_reg with CombineLd; k_combine otherwise)
+ *                      register Stockham pass (FP32 k_fft_pair, FP64 k_fft_reg, with
+ *                      CombineLd; k_combine otherwise)
  *                      (:956-968 and the MPI_Alltoall of :970)
- *   9  size-M FFTs     register Stockham passes k_fft_reg (k_fft_pass for shapes they do not
- *                      take) (FFTW at :1080)
+ *   9  size-M FFTs     register Stockham passes, FP32 k_fft_pair, FP64 k_fft_reg (k_fft_pass for
+ *                      shapes they do not take) (FFTW at :1080)
  *  10  k_block_dc      FP32 plans: the block-DC bins from the exact identity in FP64
  *
- * Row contractions run on the tensor cores for split-TF32 plans (fmmfft_tc.cuh: k_tc_rowgemm,
- * k_tc_rowgemm16) and as rowgemm on the CUDA cores otherwise.
+ * Sections of up to a few thousand points run stages 1 to 7 in one block each (fmmfft_tree.cuh).  Row
+ * contractions: FP64 on the FP64 matrix instructions (fmmfft_rows.cuh), FP32 on the CUDA cores
+ * (fmmfft_rows32.cuh), split-TF32 and BF16x3 plans on tcgen05 where rows are long and levels large
+ * (fmmfft_tc.cuh, the leaf fmmfft_tcss.cuh) and as FP32 otherwise; rowgemm for shapes these do not take.
  * All tree operators are shared by every section and box, so each tree stage is one dense
  * contraction over "rows" (section, re/im plane, box) with a small operator; rowgemm is the
  * CUDA-core form of that contraction.  Real type R = float (complex64 plans) or double
@@ -183,9 +188,9 @@ template <typename R> struct Dev {
   long tc_min_rows; /* stages with fewer rows use the CUDA-core kernel */
   int fft_threads;  /* threads per block of the register FFT pass (power of two, <= 512) */
   /* tensor-core kernel: 0 row form (32 lanes), 3 row form (16 lanes), 4 warp-specialised; -1
-   * per stage: S2M, M2M and M2L the 16-lane row form (form_m2l), the leaf its neighbour-sum form
-   * (or the 32-lane window form).  The autotuner chooses among -1, 3 and 4; BF16x3 plans always
-   * use 4 (the only BF16x3 kernel). */
+   * per stage: S2M, M2M and M2L the 16-lane row form (form_m2l).  The leaf takes its shared-memory form
+   * (ss_leaf) whatever this says, else the neighbour-sum form (or the 32-lane window form).  The
+   * autotuner chooses among -1, 3 and 4; BF16x3 tree stages always use 4 (the only BF16x3 kernel). */
   int tc_form;
   int form_m2l; /* M2L's tensor-core form when tc_form does not force one */
   int bf16;    /* FMMFFT_BF16X3: the tensor-core stages in BF16x3 instead of split TF32 */
@@ -194,8 +199,7 @@ template <typename R> struct Dev {
   long coarse_rows; /* levels with fewer rows go to the coarse-tree kernel (0: none) */
   int coarse_grid;  /* blocks of the coarse-tree kernel an SM holds (0: its operators do not fit) */
   int fuse_s2m;     /* S2M inside the sections pass where tiles hold whole boxes */
-  /* FP64 plans: tree stages and leaf as row contractions on the FP64 matrix instructions
-   * (fmmfft_rows.cuh) and their operators */
+  /* tree stages and leaf as row contractions (fmmfft_rows.cuh, fmmfft_rows32.cuh) where no tensor-core stage has them */
   int rows;
   int tree;   /* the sections run whole in k_tree */
   R *tops;    /* operators of the row contractions and of k_tree (TreeOps) */
@@ -1952,25 +1956,26 @@ static void launch_fft_pair(const StridedLd<float> &ld, float2 *out, const float
     else k_fft_pair<false, false, StridedLd2, G><<<g, thr, sm, st>>>(ld2, out, twD, twP, fp, O);
   });
 }
-/* the shared-memory opt-in of every build */
-template <typename R, int G, int HI> static void fft_smem_limit(int lim) {
+/* The shared-memory opt-in of the builds whose blocks can need more than 48 KB: two sequences a thread from
+ * L = 512 (the combine from 128 sections), FP64 from L = 256 (128 sections), the builds for any L.  (Every opt-in
+ * loads its kernel, which a process pays once.) */
+template <typename R, int G> static void fft_smem_limit(int lim) {
   constexpr auto at = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  if constexpr (sizeof(R) == 4) {
-    if constexpr (G == 0 || (G >= kFftLo && G <= kFftHi)) {
-      cudaFuncSetAttribute(k_fft_pair<true, true, StridedLd2, G>, at, lim);
-      cudaFuncSetAttribute(k_fft_pair<true, false, StridedLd2, G>, at, lim);
-      cudaFuncSetAttribute(k_fft_pair<false, false, StridedLd2, G>, at, lim);
-    }
-    if constexpr (G == 0 || (G >= kCombLo && G <= kCombHi)) cudaFuncSetAttribute(k_fft_pair<false, false, CombineLd2, G>, at, lim);
+  if constexpr (sizeof(R) == 4 && (G == 0 || G >= 9)) {
+    cudaFuncSetAttribute(k_fft_pair<true, true, StridedLd2, G>, at, lim);
+    cudaFuncSetAttribute(k_fft_pair<true, false, StridedLd2, G>, at, lim);
+    cudaFuncSetAttribute(k_fft_pair<false, false, StridedLd2, G>, at, lim);
   }
-  if constexpr (G == 0 || (G >= kFftLo && G <= kFftHi)) {
+  if constexpr (G == 0 || (sizeof(R) == 8 && G >= 8)) {
     cudaFuncSetAttribute(k_fft_reg<R, true, true, StridedLd<R>, false, G>, at, lim);
     cudaFuncSetAttribute(k_fft_reg<R, true, false, StridedLd<R>, false, G>, at, lim);
     cudaFuncSetAttribute(k_fft_reg<R, false, false, StridedLd<R>, false, G>, at, lim);
   }
-  if constexpr (G == 0 || (G >= kCombLo && G <= kCombHi))
+  if constexpr (sizeof(R) == 4 && (G == 0 || (G >= 7 && G <= kCombHi)))
+    cudaFuncSetAttribute(k_fft_pair<false, false, CombineLd2, G>, at, lim);
+  if constexpr (G == 0 || (sizeof(R) == 8 && G >= 7 && G <= kCombHi))
     cudaFuncSetAttribute(k_fft_reg<R, false, false, CombineLd<R>, false, G>, at, lim);
-  if constexpr (G < HI) fft_smem_limit<R, G == 0 ? (kFftLo < kCombLo ? kFftLo : kCombLo) : G + 1, HI>(lim);
+  if constexpr (G < kFftHi) fft_smem_limit<R, G == 0 ? 7 : G + 1>(lim);
 }
 
 /* Launch one FFT pass: the register kernel when the shape allows it, else the shared-memory
@@ -2916,7 +2921,7 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
     }
     pf.launches[ST_S2M]++;
   }
-  /* coarse tree: levels below the row threshold run in one cooperative launch (stage 5) */
+  /* coarse tree: levels below the row threshold run in one launch (stage 5) */
   long thr = d->coarse_rows;
   if (d->tc && d->tc_min_rows < thr) thr = d->tc_min_rows; /* never take a level off the TCs */
   /* routing by the row counts of ONE transform, so that a transform takes the same kernels (and
@@ -3407,8 +3412,8 @@ static int set_smem_limits(void) {
   int lim = maxopt > 0 ? maxopt : 48 * 1024;
   cudaFuncSetAttribute(k_fft_pass<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_fft_pass<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  fft_smem_limit<float, 0, kFftHi>(lim);
-  fft_smem_limit<double, 0, kFftHi>(lim);
+  fft_smem_limit<float, 0>(lim);
+  fft_smem_limit<double, 0>(lim);
   cudaFuncSetAttribute(k_fft_reg<float, false, false, CombineLd<float>, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_fft_reg<float, true, true, StridedLd<float>, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_fft_reg<float, true, false, StridedLd<float>, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
