@@ -135,7 +135,8 @@ def stage_bytes(N, P, T, b, esz):
     xt_all = 2 * P * M * R
     xt_sec = 2 * S1 * M * R
     u = 2 * S1 * M * R
-    # levels of fewer than 4096 rows (2 (P-1) boxes each) run in the coarse-tree launch
+    # levels of fewer than 4096 rows (2 (P-1) boxes each) count to the coarse-tree launch (those of 2048
+    # rows up have launches of their own now; their bytes are under 1% of the tree's)
     coarse = lambda rows: rows < 4096
     m2m = [l for l in range(2, n)]
     m2l = [l for l in range(3, n + 1)]
@@ -158,14 +159,14 @@ def stage_bytes(N, P, T, b, esz):
 
 
 # DRAM bytes (read + write) per launch of the stage's kernel from one ncu capture of the bench
-# command (profiles/k_tc_nbr_TcLeafNb_N2p24_P64_T24_b32.txt, k_sections_f32_N2p24_P64_T24_b32.txt,
-# k_tc_rowgemm16_TcM2L_N2p24_P64_T24_b32.txt).  M2L: the finest of its seven launches was captured
-# (213.4 MB for 2^12 parents per section plane); the mean over the seven levels scales it by the
-# levels' rows, (2^13 - 2^6) / 2^12 / 7.  Only meaningful for the headline workload.
+# command (profiles/k_tc_ss_TcLeafSs_N2p24_P64_T24_b32.txt, k_sections_f32_N2p24_P64_T24_b32.txt,
+# k_tc_rowgemm16_TcM2L_N2p24_P64_T24_b32.txt).  M2L: the finest of its eight launches was captured
+# (213.4 MB for 2^12 parents per section plane); the mean over the eight levels scales it by the
+# levels' rows, (2^13 - 2^5) / 2^12 / 8.  Only meaningful for the headline workload.
 TRAFFIC_PER_LAUNCH = {
-    "leaf_l2t_near": 240.520704e6 + 98.922752e6,
+    "leaf_l2t_near": 236.479744e6 + 96.224512e6,
     "sections": 134.243840e6 + 186.710528e6,
-    "m2l_l2l": (148.727808e6 + 64.687360e6) * ((1 << 13) - (1 << 6)) / (1 << 12) / 7,
+    "m2l_l2l": (148.727808e6 + 64.687360e6) * ((1 << 13) - (1 << 5)) / (1 << 12) / 8,
 }
 
 

@@ -56,9 +56,10 @@ typedef enum {
                          the transform (7e-5 relative at P = 64), while its truncation there is
                          below 3.3e-8 for terms >= 10.  FP64 plans keep the FMM's value. */
   FMMFFT_F32_TC = 2,  /* operator contractions on tcgen05 tensor cores in split TF32 (operands
-                         split into TF32 hi + lo, three products, FP32 accumulation), rest FP32 */
-  FMMFFT_BF16X3 = 3   /* the same contractions in BF16x3 (BF16 hi + lo, three products, FP32
-                         accumulation, ~2^-17 per product): for orders whose truncation error is
+                         split into TF32 hi + lo, FP32 accumulation) where they are faster than in
+                         FP32 (the leaf; tree stages of many terms), rest FP32 */
+  FMMFFT_BF16X3 = 3   /* the tree's contractions in BF16x3 (BF16 hi + lo, three products, FP32
+                         accumulation, ~2^-17 per product), the leaf in split TF32: for orders whose truncation error is
                          well above 1e-5 (the 1e-4 accuracy class); rest FP32 */
 } fmmfft_precision;
 
