@@ -1918,7 +1918,7 @@ template <int LO, int HI, class F> static void fft_by_len(int L, F f) {
     else fft_by_len<LO + 1, HI>(L, f);
   }
 }
-constexpr int kFftLo = 6, kFftHi = 10, kCombLo = 4, kCombHi = 8;
+constexpr int kFftLo = 6, kFftHi = 11, kCombLo = 4, kCombHi = 8;
 template <typename R>
 static void launch_fft_reg(const StridedLd<R> &ld, typename cplx<R>::T *out, const typename cplx<R>::T *twD,
                            const typename cplx<R>::T *twP, const FftPass &fp, bool tin, bool tout, dim3 g, int thr, size_t sm,
@@ -4297,9 +4297,11 @@ extern "C" int fmmk_fft_create(long N, int dbl, fmmk_fft **out, size_t *device_b
     f->npass = 1;
     f->pass[0] = plain_pass((int)N, 1, N, N, 1, N, N, 1, 0, 1, N);
     f->per[0] = 1, f->rows[0] = 1, f->tin[0] = 1, f->tout[0] = 1, f->src[0] = 0, f->dst[0] = 1;
-  } else if (lg <= 21) {
-    int a = lg / 2 > 9 ? 9 : lg / 2;
-    if (a < lg - 12) a = lg - 12;
+  } else if (lg <= 22) {
+    /* Two passes while both lengths stay at 2^11: a block then has 4 sequences, 32-byte pieces, which cost less
+     * than a third pass (2^22, us: FP32 79 -> 65, FP64 161 -> 142).  Below 2^21 a first pass of at most 2^9, so that its
+     * pieces are longer (FP64 2^20: 40, with 2^10 42; 2^21 85, with 2^10 77). */
+    const int a = lg >= 21 || lg / 2 <= 9 ? lg / 2 : 9;
     const long N2 = 1L << a, N1 = N / N2;
     f->npass = 2;
     /* for each n1: DFT over n2 (stride N1), times exp(-2 pi i n1 k2 / N) -> tmp[k2 N1 + n1] */
