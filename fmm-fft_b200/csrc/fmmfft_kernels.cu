@@ -1359,7 +1359,8 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 1) k_leaf(const R *_
  * weight serves the re and im planes: 128 FMAs for 16 (FP64) shared 16-byte loads.  The shares'
  * sums are added in a fixed order with the far field.  Bound by the FP64 unit (N = 2^16, P = 4, b = 2048:
  * 604 M FMAs, 36 us at its rate): 72 us there against k_leaf's 494 on 48 blocks; 64 targets a block
- * measured 80.  Grid (M / 128, P - 1, transforms). */
+ * measured 80.  With few blocks of k_leaf it is the faster one at every width (b 128 to 2048, FP32 and FP64,
+ * up to 32000 rows: 0.06 to 0.82 of k_leaf's time).  Grid (M / 128, P - 1, transforms). */
 constexpr int kWideMin = 128, kWideTgt = 128, kWideSrc = 1024; /* least b; targets, points at a time */
 template <typename R>
 __global__ void __launch_bounds__(256) k_leaf_wide(const R *__restrict__ psi_n, const R *__restrict__ xt,
@@ -2779,6 +2780,24 @@ template <typename R> static void dev_release(Dev<R> *d) {
   delete d;
 }
 
+/* Where a plan's leaf multipoles come from; the shape of ONE transform decides, so that a transform takes
+ * the same kernel alone and in a batch.  From rows enough for the tensor cores on they go there.  Wide
+ * boxes (b >= kWideMin): k_s2m_wide's time grows with rows b, the row contraction's (128 rows a block) is
+ * constant, and grows with b, until its blocks fill the device.  The two cross near 30 b rows while boxes
+ * are narrow, near 12000 rows on 148 SMs from b = 512 on (T 8 to 24, us row contraction / k_s2m_wide: FP32
+ * b = 128, 16 terms: 1984 rows 53 / 28, 4032 51 / 50, 8064 51 / 94, 16128 51 / 179; FP64 b = 256: 4032 65 /
+ * 42, 8064 75 / 77; FP64 b = 512, 24 terms: 8160 rows 0.72 of the time). */
+enum S2mRoute { S2M_FUSED, S2M_ROWS, S2M_TC, S2M_WIDE, S2M_GENERAL };
+static const char *const kS2mNames[] = {"fused", "rows", "tensor_cores", "wide", "general"};
+template <typename R> static S2mRoute s2m_route(const Dev<R> *d) {
+  const long rows = 2 * d->S1 * d->s, b = d->b;
+  const bool on_rows = d->rows, on_tc = sizeof(R) == 4 && d->tc && d->ok_s2m && rows >= d->tc_min_rows;
+  if (d->tileM % b == 0 && d->T % 4 == 0 && d->fuse_s2m && !(on_rows && sizeof(R) == 8)) return S2M_FUSED;
+  if (on_tc) return S2M_TC;
+  if (on_rows) return S2M_ROWS;
+  return b >= kWideMin && rows < 24 * b && rows < 64L * d->num_sms ? S2M_WIDE : S2M_GENERAL;
+}
+
 /* Parts of one execute (a shard of a sharded transform runs its plan's stages in pieces, with
  * exchanges between them); a null control runs the whole transform. */
 struct ExecCtl {
@@ -2855,7 +2874,8 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
   /* 1-2: sections and their sums */
   stage(ST_SECTIONS);
   /* S2M fused into the sections pass when tiles hold whole leaf boxes */
-  const bool s2m_fused = d->tileM % b == 0 && T % 4 == 0 && d->fuse_s2m && !(d->rows && sizeof(R) == 8);
+  const S2mRoute s2m = s2m_route(d);
+  const bool s2m_fused = s2m == S2M_FUSED;
   if (run(ST_SECTIONS)) {
     int TMt = (int)d->tileM;
     size_t sm = sizeof(C) * TMt * (P + 1) + (s2m_fused ? sizeof(R) * b * T : 0);
@@ -2881,42 +2901,31 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
   /* 3: S2M at level n (done in stage 1 when fused) */
   stage(ST_S2M);
   if (!s2m_fused && run(ST_S2M)) {
-    bool done = false;
     const long rows1 = 2 * S1 * s;
     R *const phi_n = d->phi + lvl_off(n, S1e, T);
-    if constexpr (sizeof(R) == 8)
-      if (d->rows) {
+    if (s2m == S2M_ROWS) {
+      if constexpr (sizeof(R) == 8)
         launch_rows(RowsS2M{d->xt, rop.s2m, phi_n, rows1, M, (int)T, (int)b, (int)P}, nbt,
                     (int)b * rows_npad((int)T), 0, d->num_sms, st, d->pdl);
-        done = true;
-      }
-    if constexpr (sizeof(R) == 4)
-      if (d->rows && !(d->ok_s2m && rows1 >= d->tc_min_rows)) {
+      else
         launch_rows32(R32S2M{d->xt, rop.s2m, phi_n, rows1, M, (int)T, (int)b, (int)P}, nbt, (int)b * EngF32::npad((int)T), 0,
                       d->num_sms, st, d->pdl);
-        done = true;
-      }
-    /* wide boxes whose row contraction (128 rows a block) would not fill the device */
-    if (!done && b >= kWideMin && rows1 < 128L * d->num_sms) {
-      k_s2m_wide<R><<<dim3((unsigned)rows1, (unsigned)nbt), kS2mThreads, 0, st>>>(d->xt, d->initch, phi_n, rows1, M, (int)T,
-                                                                          (int)b, (int)P);
-      done = true;
-    }
-    if constexpr (sizeof(R) == 4) {
-      if (!done && d->tc && d->ok_s2m && rows1 >= d->tc_min_rows) {
+    } else if (s2m == S2M_TC) {
+      if constexpr (sizeof(R) == 4) {
         TcS2M q{};
-        q.rows = 2 * S1 * s, q.batches = nbt, q.nchunks = 1, q.clen[0] = (int)b, q.coff[0] = 0;
+        q.rows = rows1, q.batches = nbt, q.nchunks = 1, q.clen[0] = (int)b, q.coff[0] = 0;
         q.P = (int)P;
         q.kpad = d->kp_s2m, q.npad = d->np_s2m, q.nout = (int)T;
         q.bimg = d->tc_s2m[0], q.bimg16 = d->tc_s2m[1], q.bimg_stride = q.bimg16_stride = 0;
         q.wsb = d->ws_s2m, q.wsb_stride = 0;
         q.xt = d->xt, q.out = d->phi + lvl_off(n, S1e, T), q.M = M, q.b = (int)b, q.T = (int)T;
         launch_tc(q, d->num_sms, d->status, st, d->tc_form < 0 ? 3 : d->tc_form, d->pdl, d->bf16);
-        done = true;
       }
-    }
-    if (!done) {
-      ProbS2M<R> pb{d->xt, d->initch, d->phi + lvl_off(n, S1e, T), 2 * S1 * s, M, (int)b, (int)T, (int)P};
+    } else if (s2m == S2M_WIDE) {
+      k_s2m_wide<R><<<dim3((unsigned)rows1, (unsigned)nbt), kS2mThreads, 0, st>>>(d->xt, d->initch, phi_n, rows1, M, (int)T,
+                                                                          (int)b, (int)P);
+    } else {
+      ProbS2M<R> pb{d->xt, d->initch, phi_n, rows1, M, (int)b, (int)T, (int)P};
       launch_rowgemm<R>(pb, pb.rows, (int)T, nbt, st);
     }
     pf.launches[ST_S2M]++;
@@ -4004,18 +4013,18 @@ extern "C" int fmmk_selftest_wait(fmmk_state *st, int which, long limit_us, char
 extern "C" int fmmk_describe(fmmk_state *st, char *buf, size_t len) {
   if (st->precision == 0) {
     Dev<double> *d = (Dev<double> *)st->dev;
-    snprintf(buf, len, "fft_threads=%d coarse_rows=%ld fuse_s2m=%d tuned=0", d->fft_threads, d->coarse_rows,
-             d->fuse_s2m);
+    snprintf(buf, len, "fft_threads=%d coarse_rows=%ld fuse_s2m=%d%s%s%s tuned=0", d->fft_threads, d->coarse_rows,
+             d->fuse_s2m, d->tree ? "" : " s2m=", d->tree ? "" : kS2mNames[s2m_route(d)], d->tree ? " sections=one_block" : "");
   } else {
     Dev<float> *d = (Dev<float> *)st->dev;
     const char *form = d->tc_form == 0 ? "row" : d->tc_form == 3 ? "row16" : d->tc_form == 4 ? "ws" : "per_stage";
     snprintf(buf, len,
              "fft_threads=%d coarse_rows=%ld tc_min_rows=%ld fuse_s2m=%d tensor_cores=%s tc_form=%s "
-             "leaf_form=%s%s tuned=%d",
+             "leaf_form=%s%s%s%s tuned=%d",
              d->fft_threads, d->coarse_rows, d->tc_min_rows, d->fuse_s2m,
              d->tc ? (d->bf16 ? "bf16x3" : "tf32x3") : "none", form,
              !d->tc || d->tree ? "cuda_cores" : d->ss_leaf ? "shared_operands" : (d->ok_lnb && d->tc_form < 0) ? "neighbour_sum" : d->ok_leaf ? "window_rows" : "cuda_cores",
-             d->tree ? " sections=one_block" : "", d->tuned);
+             d->tree ? "" : " s2m=", d->tree ? "" : kS2mNames[s2m_route(d)], d->tree ? " sections=one_block" : "", d->tuned);
   }
   return 0;
 }
