@@ -201,7 +201,8 @@ template <typename R> struct Dev {
   int fuse_s2m;     /* S2M inside the sections pass where tiles hold whole boxes */
   /* tree stages and leaf as row contractions (fmmfft_rows.cuh, fmmfft_rows32.cuh) where no tensor-core stage has them */
   int rows;
-  int tree;   /* the sections run whole in k_tree */
+  int tree;   /* the sections run whole in k_tree, tree_blocks blocks of 128 threads an SM */
+  int tree_blocks;
   R *tops;    /* operators of the row contractions and of k_tree (TreeOps) */
   TreeStage *tstages; /* k_tree's stages: with resident operators, with operators in turn */
   unsigned env_set; /* knobs an environment switch fixed (the autotuner leaves them): bits below */
@@ -2405,18 +2406,29 @@ template <typename R> static void coarse_setup(Dev<R> *d) {
   if (d->coarse_grid < 1) d->coarse_rows = 0; /* operator too large for shared memory */
 }
 
-/* Whether the plan's sections run whole in one block (k_tree): FP32 plans (split-TF32 and BF16x3 ones
- * too, whose tree stages are below the tensor cores' row threshold there) up to what shared memory
- * holds, FP64 ones up to 1024 points a section.  Measured, k_tree against a launch per stage, us a
- * transform: FP32, 20 terms, P = 64: one of 2^16 39 / 45, 2^18 70 / 92, 16 of 2^16 120 / 322, 4 of 2^18
- * (split TF32) 127 / 197; FP64, 16 terms: 16 of 2^16 144 / 232, but 16 of 2^17 345 / 308, where the row
- * contractions fill the device.  The choice depends on the shape alone, so that a transform takes the
- * same kernel alone and in a batch.  A switch that steers the stage kernels keeps those. */
-constexpr long kTreeMaxF64 = 1024;
+/* Whether the plan's sections run whole in one block (k_tree).  FP64 plans: up to 1024 points a section
+ * (16 terms: 16 of 2^16 144 us in one block / 232 in stages, 16 of 2^17 345 / 308, where the row contractions
+ * fill the device).  FP32 plans of every kind: where the sections of one transform, P blocks, are on the
+ * device at once, with twice as many where the stages lack the FP32 row contractions for their large levels
+ * (more than 32 terms; BF16x3), and above 512 sections only up to 32 points each.  More sections than
+ * that lose to the stages, alone and in a batch (us, one block / stages, split TF32, b = 32: P = 512 of 4096
+ * points, 24 terms 402 / 179; P = 256 of 4096, 16 terms, 4 transforms 545 / 234; P = 1024 of 256, 24 terms, 16
+ * transforms 614 / 441); fewer win alone (P = 64 of 1024, 20 terms 39 / 45).  Over 1550 shapes and
+ * batches the rule's transforms take 0.92 of the time of one block wherever it fits, none more than when
+ * there were only stages.  The choice depends on the shape alone, so that a transform takes the same kernel
+ * alone and in a batch.  A switch that steers the stage kernels keeps those. */
+constexpr long kTreeMaxF64 = 1024, kTreeSms = 148; /* SMs of the device: a constant, a shape's route is fixed */
+static bool tree_one_wave(long M, long P, int blocks, bool no_rows) {
+  return P > 512 ? M <= 32 : P <= kTreeSms * blocks * (no_rows ? 2 : 1);
+}
 template <typename R> static void tree_setup(Dev<R> *d) {
   using E = typename TreeEng<R>::E;
   const int T = (int)d->T, b = (int)d->b, n = (int)d->n;
-  d->tree = b >= 8 && b <= 64 && n <= kTreeMaxLevel && (sizeof(R) == 4 || d->M <= kTreeMaxF64) &&
+  if (n > kTreeMaxLevel) return;
+  /* blocks of 128 threads that an SM holds: by shared memory, at most the five that registers allow */
+  const size_t sm = tree_smem<E>(T, b, n, 0) + 1024;
+  d->tree_blocks = sm * 5 <= (size_t)227 * 1024 ? 5 : (int)((size_t)227 * 1024 / sm);
+  d->tree = b >= 8 && b <= 64 && (sizeof(R) == 4 ? tree_one_wave(d->M, d->P, d->tree_blocks, T > 32 || d->bf16) : d->M <= kTreeMaxF64) &&
             !(d->env_set & (KNOB_COARSE | KNOB_TCMIN | KNOB_FUSE | KNOB_FORM)) && !getenv("FMMFFT_TC_STAGES") &&
             !getenv("FMMFFT_LEAF_FORM") && tree_smem<E>(T, b, n, 0) <= (size_t)200 * 1024;
 }
@@ -2858,9 +2870,10 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
   if (d->tree && !ctl) { /* 1-7 in one launch, a block per section */
     using E = typename TreeEng<R>::E;
     stage(ST_SECTIONS);
-    /* blocks enough to fill the device: large tiles, small blocks and one operator at a time; else all
-     * operators copied at the start and small tiles on more threads */
-    const bool many = P * nbt > 2L * d->num_sms;
+    /* blocks enough to fill the device, several an SM: large tiles, small blocks and one operator at a time;
+     * else small tiles on more threads, with all operators copied at the start where they fit (16 of 2^18, P = 64,
+     * 16 terms, one block an SM: 339 us on 512 threads, 542 on 128) */
+    const bool many = P * nbt > 2L * d->num_sms && d->tree_blocks > 1;
     const int resident = !many && tree_smem<E>((int)T, (int)b, (int)n, 1) <= (size_t)200 * 1024;
     const TreeArgs<E> ta{x, d->xt, d->ssum, d->phi, d->psi, d->u, rop, d->evalmh, d->cot,
                          d->tstages + (resident ? 0 : kTreeStages), M, S1e, (int)P, (int)T, (int)b, (int)n, inverse,
