@@ -94,7 +94,7 @@ struct RowsS2M {
 };
 
 /* Leaf of section z + 1 (reference src/fmmfft.c:751-954): rows (transform, plane, box), segments
- * psi[box], x[box - 1], x[box], x[box + 1].  For sc >= P/2 a box's first point lies in the box before
+ * psi[box], x[box - 1], x[box + 1] and, its weights reach P / pi, last x[box].  For sc >= P/2 a box's first point lies in the box before
  * it (half-shifted): its value is that of the expansion and the window one box earlier with the
  * weights evalmh and cot[0 .. 3b), or for sc = P/2 the mean of both. */
 struct RowsLeaf {
@@ -116,7 +116,7 @@ struct RowsLeaf {
     p[1] = x + ((bx - 1) & (s - 1)) * b, p[2] = x + (bx & (s - 1)) * b, p[3] = x + ((bx + 1) & (s - 1)) * b;
   }
   __device__ void base(long r, int z, const double *(&p)[NP]) const { window(r, z, 0, p); }
-  static __device__ __forceinline__ const double *seg(const double *const (&p)[NP], int g, int) { return p[g]; }
+  static __device__ __forceinline__ const double *seg(const double *const (&p)[NP], int g, int) { return p[g < 2 ? g : 5 - g]; }
   __host__ __device__ int ncol() const { return b; }
   __device__ double *dst(long r, int, int z) const { return u + plane(r, z) * M + (r & (s - 1)) * b; }
 };
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(kRowsThreads, 3) k_rows_f64(const __grid_const
         for (int i = 0; i < RT; ++i)
 #pragma unroll
           for (int j = 0; j < NT; ++j) acc[q][i][j][0] = acc[q][i][j][1] = 0.0;
-      int sofs = 0; /* leaf: the segment's block */
+      int sofs = 0; /* leaf: the segment's block (the operator has them in box order) */
 #pragma unroll
       for (int s = 0; s < Prob::NSEG; ++s) {
         const int len = pb.len(s), k4n = (len + 3) >> 2, bsz = k4n * nt * 32;
@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(kRowsThreads, 3) k_rows_f64(const __grid_const
         const double *bq[Prob::NPAR];
 #pragma unroll
         for (int q = 0; q < Prob::NPAR; ++q) {
-          if constexpr (Prob::kLeaf) bq[q] = sop + sofs + j0 * 32 + lane;
+          if constexpr (Prob::kLeaf) bq[q] = sop + sofs + (s == 2 ? bsz : s == 3 ? -bsz : 0) + j0 * 32 + lane;
           else bq[q] = sop + Prob::blk(q, s) * bsz + j0 * 32 + lane;
         }
         sofs += bsz;
