@@ -180,7 +180,7 @@ template <typename R> struct Dev {
    * core-matrix layout (tc::ws_b_index), one block per level or section */
   float *ws_s2m, *ws_m2m, *ws_m2l, *ws_leaf;
   long ws_m2m_stride, ws_m2l_stride, ws_leaf_stride;
-  int Tk;           /* K positions of an expansion in the leaf's operator: T rounded up to 8 */
+  int Tk;           /* K positions of an expansion in the leaf's operator: T, in the shared-memory form rounded up to 8 */
   int ss_leaf;      /* stages of the leaf's shared-memory form (tc::k_tc_ss), 0: not used */
   int kp_s2m, np_s2m, kp_m2m, np_m2m, kp_m2l, np_m2l, kp_leaf, np_leaf;
   int ok_s2m, ok_m2m, ok_m2l, ok_leaf;
@@ -2470,9 +2470,9 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
   d->tc = tc;
   d->kp_s2m = up8(b), d->np_s2m = up16(T);
   d->kp_m2m = up8(2 * T), d->np_m2m = up16(T);
-  d->Tk = up8(T); /* the leaf's segments of K start on a K step */
   d->kp_m2l = up8(5 * T), d->np_m2l = up16(2 * T);
-  d->kp_leaf = up8(d->Tk + 3 * b), d->np_leaf = up16(b + 1); /* + the half-shifted column */
+  d->Tk = (int)T;
+  d->kp_leaf = up8(T + 3 * b), d->np_leaf = up16(b + 1); /* + the half-shifted column */
   d->kp_lnb = up8(T + b), d->np_lnb = up16(3 * b + 3);    /* three blocks + three half-shift columns */
   auto fits = [&](int kp, int np) {
     return tc && (T % 4 == 0) && (b % 4 == 0) && np <= 256 && kp <= 256 &&
@@ -2543,8 +2543,10 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
   using E = typename TreeEng<R>::E;
   /* The leaf's shared-memory form: whole tiles of 128 boxes, unless a switch steers the stage kernels.  It is
    * the faster one at every size with them (2^20 T20, P64: 31 us -> 24; 2^26 T16, P256: 860 -> 648). */
-  if (tc && d->ok_leaf && b % 8 == 0 && s >= tc::kRows && !steered)
-    d->ss_leaf = ss_stages(d->kp_leaf, d->np_leaf, (int)(d->Tk + b) / 4, (int)b);
+  if (tc && d->ok_leaf && b % 8 == 0 && s >= tc::kRows && !steered) {
+    d->ss_leaf = ss_stages(d->kp_leaf, d->np_leaf, (up8(T) + (int)b) / 4, (int)b);
+    if (d->ss_leaf) d->Tk = up8(T); /* kp_leaf has room for it: b is a multiple of 8 */
+  }
   if (!shard) tree_setup<R>(d); /* a shard runs its stages in pieces */
   if (d->tree) d->ok_s2m = d->ok_m2m = d->ok_m2l = d->ok_leaf = d->ok_lnb = 0; /* no stage reaches them */
   /* a small level's row contraction costs 3 to 4 us, less than the same level in the coarse tree from
