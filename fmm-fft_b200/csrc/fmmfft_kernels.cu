@@ -2206,9 +2206,6 @@ static float bf16_to_float_host(uint16_t b) {
   return f;
 }
 
-/* Uploads one operator, given as FP64 [npad][kpad] K-major values, split into TF32 hi and lo:
- * as two [npad][kpad] arrays (dhi, dlo) and, when dws is given, as the warp-specialised
- * kernel's block (hi rows 0..npad-1, lo rows npad..2 npad-1, core-matrix layout). */
 /* Splits operator v ([npad][kpad], row n = output column n, zero padded) into TF32 hi / lo and
  * uploads the images the kernels copy into shared memory as they are:
  *   dimg   the row forms' (k_tc_rowgemm, k_tc_nbr): hi rows then lo rows, K-major core
@@ -2236,6 +2233,7 @@ static int tc_put(float *dimg, float *dimg16, float *dws, const double *v, int k
     const long o = (long)(tc::core_off(n, k, kpad) >> 2);
     img[o] = h[i];
     img[cnt + o] = h[cnt + i];
+    if (!dws) continue;
     if (bf16) {
       const uint16_t bh = bf16_rne_host(f);
       const float fh = bf16_to_float_host(bh);
@@ -2246,7 +2244,7 @@ static int tc_put(float *dimg, float *dimg16, float *dws, const double *v, int k
       w[tc::ws_b_index(npad + n, k, kpad)] = h[cnt + i];
     }
   }
-  for (int n = 0; n < npad; ++n)
+  for (int n = 0; n < (dimg16 ? npad : 0); ++n)
     for (int k = 0; k < kp16; ++k) {
       const int ks = tc::perm16(k);
       const long o = (long)(tc::core_off(n, k, kp16) >> 2), src = (long)tc::perm16(n) * kpad + ks;
@@ -2344,8 +2342,9 @@ template <typename R> static int tc_upload_ops(Dev<R> *d, const fmm_ops64 *o, ch
         for (long k = 0; k < T; ++k) v[b * kp + k] = o->evalmh[(sc - P / 2) * T + k];
         for (long q = 0; q < 3 * b; ++q) v[b * kp + Tk + q] = ct[q];
       }
-      rc |= tc_put(d->tc_leaf[0] + (sc - 1) * 2 * d->tc_leaf_stride, d->tc_leaf[1] + (sc - 1) * d->tc_leaf_stride16,
-                   d->ws_leaf + (sc - 1) * d->ws_leaf_stride, v, kp, np, err, errlen, d->bf16);
+      rc |= tc_put(d->tc_leaf[0] + (sc - 1) * 2 * d->tc_leaf_stride,
+                   d->tc_leaf[1] ? d->tc_leaf[1] + (sc - 1) * d->tc_leaf_stride16 : nullptr,
+                   d->ws_leaf ? d->ws_leaf + (sc - 1) * d->ws_leaf_stride : nullptr, v, kp, np, err, errlen, d->bf16);
     }
   if (d->ok_lnb && w01) /* neighbour-sum form (TcLeafNb): x_B's weights for boxes B, B+1, B-1 */
     for (long sc = 1; sc < P; ++sc) {
@@ -2548,7 +2547,11 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
     if (d->ss_leaf) d->Tk = up8(T); /* kp_leaf has room for it: b is a multiple of 8 */
   }
   if (!shard) tree_setup<R>(d); /* a shard runs its stages in pieces */
-  if (d->tree) d->ok_s2m = d->ok_m2m = d->ok_m2l = d->ok_leaf = d->ok_lnb = 0; /* no stage reaches them */
+  /* a form that no stage reaches gets no operators: one block a section, or a leaf in the shared-memory form,
+   * whatever the tuner takes for the other stages (2^24, P = 64, 24 terms: 10 MB, 170 KB a section) */
+  if (d->tree) d->ok_s2m = d->ok_m2m = d->ok_m2l = d->ok_leaf = d->ok_lnb = d->ss_leaf = 0;
+  if (d->ss_leaf) d->ok_lnb = 0;
+  const bool leaf_rows = d->ok_leaf && !d->ss_leaf; /* the leaf's 16-lane and warp-specialised forms */
   /* a small level's row contraction costs 3 to 4 us, less than the same level in the coarse tree from
    * about 1024 rows in FP64 and 2048 in FP32 (levels from 1024 / 2048 / 4096 rows, us a transform: FP64 2^20, P =
    * 32, 15 terms 145 / 148 / 146; FP32 2^20, P = 64, 20 terms 123 / 121 / 123; split TF32 2^24, 24 terms 816 / 819 /
@@ -2576,7 +2579,7 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
   const long ws_s2m_n = d->ok_s2m ? (long)tc::ws_b_floats(d->kp_s2m, d->np_s2m) / wdiv : 0;
   const long ws_m2m_n = d->ok_m2m ? nlev * d->ws_m2m_stride : 0;
   const long ws_m2l_n = d->ok_m2l ? nlev * d->ws_m2l_stride : 0;
-  const long ws_leaf_n = d->ok_leaf ? S1 * d->ws_leaf_stride : 0;
+  const long ws_leaf_n = leaf_rows ? S1 * d->ws_leaf_stride : 0;
   size_t off = 0;
 #define CARVE(field, count, type)          \
   size_t off_##field = off;                \
@@ -2612,7 +2615,7 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
   CARVE(tcs2m16, d->ok_s2m ? d->tc_s2m_stride16 : 0, float)
   CARVE(tcm2m16, d->ok_m2m ? nlev * d->tc_m2m_stride16 : 0, float)
   CARVE(tcm2l16, d->ok_m2l ? nlev * d->tc_m2l_stride16 : 0, float)
-  CARVE(tcleaf16, d->ok_leaf ? S1 * d->tc_leaf_stride16 : 0, float)
+  CARVE(tcleaf16, leaf_rows ? S1 * d->tc_leaf_stride16 : 0, float)
   CARVE(leaffix, (d->ok_leaf || d->ok_lnb) ? nb * 2 * s : 0, float)
   CARVE(lnbw, (d->ok_lnb || d->ok_leaf) ? 2 * S1 : 0, float)
   CARVE(wss2m, ws_s2m_n, float)
@@ -2620,7 +2623,8 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
   CARVE(wsm2l, ws_m2l_n, float)
   CARVE(wsleaf, ws_leaf_n, float)
   CARVE(tstages, d->tree ? 2 * kTreeStages : 0, TreeStage)
-  const long ntops = tree_nops<E>(d->rows || d->tree ? P : 1, T, b, nlev); /* the leaf's for row contractions only */
+  const bool leaf_ops = (d->rows && !d->ss_leaf) || d->tree; /* else the tree stages' only */
+  const long ntops = tree_nops<E>(leaf_ops ? P : 1, T, b, nlev);
   CARVE(tops, ntops, R)
 #undef CARVE
   if (dry_bytes) {
@@ -2664,14 +2668,14 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
   d->tc_s2m[0] = (float *)(base + off_tcs2m), d->tc_s2m[1] = (float *)(base + off_tcs2m16);
   d->tc_m2m[0] = (float *)(base + off_tcm2m), d->tc_m2m[1] = (float *)(base + off_tcm2m16);
   d->tc_m2l[0] = (float *)(base + off_tcm2l), d->tc_m2l[1] = (float *)(base + off_tcm2l16);
-  d->tc_leaf[0] = (float *)(base + off_tcleaf), d->tc_leaf[1] = (float *)(base + off_tcleaf16);
+  d->tc_leaf[0] = (float *)(base + off_tcleaf), d->tc_leaf[1] = leaf_rows ? (float *)(base + off_tcleaf16) : nullptr;
   d->tc_lnb[0] = (float *)(base + off_tclnb), d->tc_lnb[1] = nullptr;
   d->leaf_fix = (float *)(base + off_leaffix);
   d->lnb_w01 = (float *)(base + off_lnbw);
   d->ws_s2m = (float *)(base + off_wss2m);
   d->ws_m2m = (float *)(base + off_wsm2m);
   d->ws_m2l = (float *)(base + off_wsm2l);
-  d->ws_leaf = (float *)(base + off_wsleaf);
+  d->ws_leaf = leaf_rows ? (float *)(base + off_wsleaf) : nullptr;
   d->tops = (R *)(base + off_tops), d->tstages = (TreeStage *)(base + off_tstages);
   cudaMemset(d->status, 0, sizeof(int));
   {
