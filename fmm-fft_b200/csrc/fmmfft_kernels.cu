@@ -2766,8 +2766,10 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
     }
     k_tree_ops<E><<<2 * d->num_sms, 256>>>(d->tops, d->initch, d->bm2m, d->bm2l, d->btop, d->evalmT, d->cot,
                                            ntops, (int)T, (int)b, (int)nlev);
-    if (cudaStreamSynchronize(0) != cudaSuccess) { /* the plan's executes may run on any stream */
-      snprintf(err, errlen, "operator layout: %s", cudaGetErrorString(cudaGetLastError()));
+    ce = cudaGetLastError(); /* a refused launch */
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(0); /* the plan's executes may run on any stream */
+    if (ce != cudaSuccess) {
+      snprintf(err, errlen, "operator layout: %s", cudaGetErrorString(ce));
       rc = 3;
     }
   }
