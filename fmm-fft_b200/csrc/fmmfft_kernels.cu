@@ -4039,13 +4039,15 @@ extern "C" int fmmk_describe(fmmk_state *st, char *buf, size_t len) {
   } else {
     Dev<float> *d = (Dev<float> *)st->dev;
     const char *form = d->tc_form == 0 ? "row" : d->tc_form == 3 ? "row16" : d->tc_form == 4 ? "ws" : "per_stage";
+    char stages[24] = ""; /* of the shared-operand leaf: tiles of samples in shared memory at once */
+    if (d->ss_leaf) snprintf(stages, sizeof stages, " leaf_stages=%d", d->ss_leaf);
     snprintf(buf, len,
              "fft_threads=%d coarse_rows=%ld tc_min_rows=%ld fuse_s2m=%d tensor_cores=%s tc_form=%s "
-             "leaf_form=%s%s%s%s tuned=%d",
+             "leaf_form=%s%s%s%s%s tuned=%d",
              d->fft_threads, d->coarse_rows, d->tc_min_rows, d->fuse_s2m,
              d->tc ? (d->bf16 ? "bf16x3" : "tf32x3") : "none", form,
              !d->tc || d->tree ? "cuda_cores" : d->ss_leaf ? "shared_operands" : (d->ok_lnb && d->tc_form < 0) ? "neighbour_sum" : d->ok_leaf ? "window_rows" : "cuda_cores",
-             d->tree ? "" : " s2m=", d->tree ? "" : kS2mNames[s2m_route(d)], d->tree ? " sections=one_block" : "", d->tuned);
+             stages, d->tree ? "" : " s2m=", d->tree ? "" : kS2mNames[s2m_route(d)], d->tree ? " sections=one_block" : "", d->tuned);
   }
   return 0;
 }
