@@ -710,7 +710,7 @@ struct TcLeafSs : TcLeaf {
   }
   /* The samples that the FP32 terms of a warp's rows need: lane's four columns c of row k = lane / cpr,
    * + rpi, .. of MMA rows 32 q .. (row m is box 16 (m % 8) + m / 8 of the tile), and the sample before
-   * the row's first.  Up to kSide loads ahead (b <= 32: all of them). */
+   * the row's first: kSide loads for b = 32, wider boxes do not fit this form. */
   static constexpr int kSide = 8;
   struct Side {
     float4 x[kSide];
@@ -747,13 +747,6 @@ struct TcLeafSs : TcLeaf {
 #pragma unroll
     for (int i = 0; i < kSide; ++i)
       if (i < cpr) row(32 * q + (lane >> lc) + i * rpi, sd.x[i], sd.prev[i]);
-    for (int i = kSide; i < cpr; ++i) {
-      const int mm = 32 * q + (lane >> lc) + i * rpi;
-      float4 x;
-      float prev;
-      side_at(abase(1, r0, z), bx0, mm, c, x, prev);
-      row(mm, x, prev);
-    }
   }
 };
 
@@ -1928,7 +1921,9 @@ static void launch_fft_reg(const StridedLd<R> &ld, typename cplx<R>::T *out, con
   fft_by_len<kFftLo, kFftHi>(fp.L, [&](auto lgt) {
     constexpr int G = decltype(lgt)::value;
     using S = StridedLd<R>;
-    if (tin && tout)
+    if constexpr (sizeof(R) == 4) /* the one-pass FFTs of single sequences and of length 16: others go in pairs */
+      k_fft_reg<R, true, true, S, false, G><<<g, thr, sm, st>>>(ld, out, twD, twP, fp, nullptr, nullptr, O);
+    else if (tin && tout)
       k_fft_reg<R, true, true, S, false, G><<<g, thr, sm, st>>>(ld, out, twD, twP, fp, nullptr, nullptr, O);
     else if (tin)
       k_fft_reg<R, true, false, S, false, G><<<g, thr, sm, st>>>(ld, out, twD, twP, fp, nullptr, nullptr, O);
@@ -1968,7 +1963,8 @@ template <typename R, int G> static void fft_smem_limit(int lim) {
     cudaFuncSetAttribute(k_fft_pair<true, false, StridedLd2, G>, at, lim);
     cudaFuncSetAttribute(k_fft_pair<false, false, StridedLd2, G>, at, lim);
   }
-  if constexpr (G == 0 || (sizeof(R) == 8 && G >= 8)) {
+  if constexpr (sizeof(R) == 4 && G == 0) cudaFuncSetAttribute(k_fft_reg<R, true, true, StridedLd<R>, false, G>, at, lim);
+  if constexpr (sizeof(R) == 8 && (G == 0 || G >= 8)) {
     cudaFuncSetAttribute(k_fft_reg<R, true, true, StridedLd<R>, false, G>, at, lim);
     cudaFuncSetAttribute(k_fft_reg<R, true, false, StridedLd<R>, false, G>, at, lim);
     cudaFuncSetAttribute(k_fft_reg<R, false, false, StridedLd<R>, false, G>, at, lim);
@@ -2003,7 +1999,7 @@ static void launch_fft_pass(const typename cplx<R>::T *in, typename cplx<R>::T *
     if (W > 16) W = 16;
     if (W > per) W = (int)per;
     if (W < 1) W = 1;
-    if (tin || W >= 4) {
+    if (sizeof(R) == 4 && !twM_lo ? tin && tout : tin || W >= 4) {
       fp.W = W;
       const StridedLd<R> sld{in, fp.M, fp.iseq, (unsigned)fp.istr};
       const int thr = W * (L / 8);
@@ -2542,7 +2538,7 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
   using E = typename TreeEng<R>::E;
   /* The leaf's shared-memory form: whole tiles of 128 boxes, unless a switch steers the stage kernels.  It is
    * the faster one at every size with them (2^20 T20, P64: 31 us -> 24; 2^26 T16, P256: 860 -> 648). */
-  if (tc && d->ok_leaf && b % 8 == 0 && s >= tc::kRows && !steered) {
+  if (tc && d->ok_leaf && b % 8 == 0 && b <= 4 * TcLeafSs::kSide && s >= tc::kRows && !steered) {
     d->ss_leaf = ss_stages(d->kp_leaf, d->np_leaf, (up8(T) + (int)b) / 4, (int)b);
     if (d->ss_leaf) d->Tk = up8(T); /* kp_leaf has room for it: b is a multiple of 8 */
   }
@@ -3228,7 +3224,8 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
         });
       }
     } else
-      fft_by_len<kCombLo, kCombHi>((int)P, [&](auto lgt) { /* a build for each usual number of sections */
+      /* a build for each usual number of sections; FP32 takes pairs from 64 sections and 8 columns on */
+      fft_by_len<kCombLo, sizeof(R) == 8 ? kCombHi : 5>((int)P, [&](auto lgt) {
         k_fft_reg<R, false, false, CombineLd<R>, false, decltype(lgt)::value>
             <<<dim3((unsigned)(ccols / Wc), (unsigned)nbt), thr, sm, st>>>(cl, cz, d->twP, d->twP, fp);
       });
