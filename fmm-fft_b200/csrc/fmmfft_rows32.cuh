@@ -28,6 +28,26 @@ struct Tile32 {
   int valid, lnb, nbt; /* rows in it; log2 of, and the rows of a plane in the tile */
 };
 
+/* cp.async of V floats (1, 2), and the rest of rows32_copy for rows that are no multiple of 4 values: copies of
+ * 8 bytes for even lengths, of 4 for odd ones.  All asynchronous: through registers a tile waited for each
+ * load in turn and M2M and the leaf lost to the general kernels (2^22, P = 64, b = 16, us M2M, M2L, leaf: 9 terms 122,
+ * 176, 93 -> 50, 90, 60, the general kernels 84, 207, 64; 10 terms 122, 177, 94 -> 45, 78, 56). */
+template <int V> __device__ __forceinline__ void cp_async_f(uint32_t dst, const float *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" : : "r"(dst), "l"(src), "n"(4 * V) : "memory");
+}
+template <int V>
+__device__ __forceinline__ void rows32_copy_by(float *dst, int pitch, const float *__restrict__ src, int first, int count, int mask,
+                                               int len) {
+  const int step = blockDim.x >> 3, np = rows_kpad(len);
+  for (int c = V * (threadIdx.x & 7); c < np; c += 8 * V)
+    for (int j = threadIdx.x >> 3; j < count; j += step) {
+      float *const d = dst + j * pitch + c;
+      if (c < len) cp_async_f<V>(tc::smem_addr(d), src + (unsigned)(((first + j) & mask) * len) + c);
+      else
+#pragma unroll
+        for (int v = 0; v < V; ++v) d[v] = 0.f;
+    }
+}
 /* `count` rows of len values, from row `first` on (wrapping at mask + 1) of the strip src, into shared
  * rows of pitch; zeros up to a multiple of 4.  Eight lanes a row. */
 __device__ __forceinline__ void rows32_copy(float *dst, int pitch, const float *__restrict__ src, int first, int count,
@@ -40,10 +60,10 @@ __device__ __forceinline__ void rows32_copy(float *dst, int pitch, const float *
       for (int j = threadIdx.x >> 3; j < count; j += step, d += 4u * step * pitch)
         tc::cp_async16(d, g + (unsigned)(((first + j) & mask) * len));
     }
+  } else if ((len & 1) == 0) {
+    rows32_copy_by<2>(dst, pitch, src, first, count, mask, len);
   } else {
-    for (int j = threadIdx.x >> 3; j < count; j += step)
-      for (int c = c8; c < rows_kpad(len); c += 8)
-        dst[j * pitch + c] = c < len ? src[(unsigned)(((first + j) & mask) * len) + c] : 0.f;
+    rows32_copy_by<1>(dst, pitch, src, first, count, mask, len);
   }
 }
 
