@@ -2796,6 +2796,10 @@ template <typename R> static void dev_release(Dev<R> *d) {
   delete d;
 }
 
+/* Shared bytes of the sections pass */
+template <typename R> static size_t sections_smem(const Dev<R> *d, bool fused) {
+  return sizeof(typename cplx<R>::T) * d->tileM * (d->P + 1) + (fused ? sizeof(R) * d->b * d->T : 0);
+}
 /* Where a plan's leaf multipoles come from; the shape of ONE transform decides, so that a transform takes
  * the same kernel alone and in a batch.  From rows enough for the tensor cores on they go there.  Wide
  * boxes (b >= kWideMin): k_s2m_wide's time grows with rows b, the row contraction's (128 rows a block) is
@@ -2808,7 +2812,9 @@ static const char *const kS2mNames[] = {"fused", "rows", "tensor_cores", "wide",
 template <typename R> static S2mRoute s2m_route(const Dev<R> *d) {
   const long rows = 2 * d->S1 * d->s, b = d->b;
   const bool on_rows = d->rows, on_tc = sizeof(R) == 4 && d->tc && d->ok_s2m && rows >= d->tc_min_rows;
-  if (d->tileM % b == 0 && d->T % 4 == 0 && d->fuse_s2m && !(on_rows && sizeof(R) == 8)) return S2M_FUSED;
+  /* the sections tile and the operator beside it in one block's shared memory */
+  const bool fits = sections_smem<R>(d, true) <= (size_t)226 * 1024;
+  if (d->tileM % b == 0 && d->T % 4 == 0 && d->fuse_s2m && fits && !(on_rows && sizeof(R) == 8)) return S2M_FUSED;
   if (on_tc) return S2M_TC;
   if (on_rows) return S2M_ROWS;
   return b >= kWideMin && rows < 24 * b && rows < 64L * d->num_sms ? S2M_WIDE : S2M_GENERAL;
@@ -2895,7 +2901,7 @@ static int dev_execute(Dev<R> *d, const void *vin, void *vout, cudaStream_t st, 
   const bool s2m_fused = s2m == S2M_FUSED;
   if (run(ST_SECTIONS)) {
     int TMt = (int)d->tileM;
-    size_t sm = sizeof(C) * TMt * (P + 1) + (s2m_fused ? sizeof(R) * b * T : 0);
+    const size_t sm = sections_smem(d, s2m_fused);
     k_sections<R><<<dim3((unsigned)d->ntile, (unsigned)nbt), 256, sm, st>>>(
         x, d->xt, d->part, M, (int)P, TMt, inverse, d->initch,
         s2m_fused ? d->phi + lvl_off(n, S1e, T) : nullptr, (int)b, (int)T, xin);

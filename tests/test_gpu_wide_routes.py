@@ -4,7 +4,8 @@ The wide kernel (a block a row) is for few rows: its time grows with rows times 
 is constant until its blocks fill the device, so plans change over at 24 b rows, and tensor-core plans from
 4096 rows keep the tensor cores.  Each shape lies near a limit: rows 4032 against 3072 (b = 128), 1984
 against 3072 and 6144, 8064 on the tensor cores.  Against the FP64 oracle of the same terms: rel-L2 <= 1e-12
-(FP64) and 1e-6 (FP32), the tolerances of the plans' other tests; a batch of two has the bits of each alone."""
+(FP64) and 1e-6 (FP32), the tolerances of the plans' other tests; a batch of two has the bits of each alone.
+P = 2 and b = 1024: the operator fits beside the sections tile up to 20 terms (FP64; FP32 48), not above."""
 import numpy as np
 import pytest
 
@@ -23,7 +24,8 @@ def fm():
 @pytest.mark.parametrize("N,P,T,b,prec,route", [
     (1 << 19, 64, 16, 128, "f32_tc", "tensor_cores"), (1 << 18, 64, 8, 128, "f32", "general"),
     (1 << 18, 64, 20, 128, "f64", "general"), (1 << 17, 32, 24, 128, "f32", "wide"),
-    (1 << 18, 32, 7, 256, "f64", "wide"), (1 << 18, 32, 12, 256, "f32_tc", "wide")])
+    (1 << 18, 32, 7, 256, "f64", "wide"), (1 << 18, 32, 12, 256, "f32_tc", "wide"),
+    (1 << 14, 2, 24, 1024, "f64", "wide"), (1 << 14, 2, 56, 1024, "f32", "wide"), (1 << 13, 2, 20, 1024, "f64", "fused")])
 def test_wide_box_multipoles(fm, monkeypatch, N, P, T, b, prec, route):
     import torch
     monkeypatch.setenv("FMMFFT_AUTOTUNE", "0")  # the default routing
