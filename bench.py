@@ -123,9 +123,17 @@ class ClockSampler:
 
 
 # ------------------------------------------------------------------------ roofline helpers
-def stage_bytes(N, P, T, b, esz):
+def coarse_rows(text):
+    """The row threshold of the plan's coarse-tree launch, from its description: its own, and never a level
+    that the tensor cores take."""
+    words = dict(w.split("=", 1) for w in text.split())
+    rows = int(words["coarse_rows"])
+    return rows if words.get("tensor_cores", "none") == "none" else min(rows, int(words["tc_min_rows"]))
+
+
+def stage_bytes(N, P, T, b, esz, rows=4096):
     """Algorithmic HBM bytes of one execute per stage: each array a stage must read or write,
-    counted once (R = esz/2 bytes per real)."""
+    counted once (R = esz/2 bytes per real); levels of fewer than `rows` rows count to the coarse-tree launch."""
     M = N // P
     S1 = P - 1
     s = M // b
@@ -135,13 +143,10 @@ def stage_bytes(N, P, T, b, esz):
     xt_all = 2 * P * M * R
     xt_sec = 2 * S1 * M * R
     u = 2 * S1 * M * R
-    # levels of fewer than 4096 rows (2 (P-1) boxes each) count to the coarse-tree launch (those of 2048
-    # rows up have launches of their own now; their bytes are under 1% of the tree's)
-    coarse = lambda rows: rows < 4096
     m2m = [l for l in range(2, n)]
     m2l = [l for l in range(3, n + 1)]
-    m2m_c = [l for l in m2m if coarse(2 * S1 * (1 << l))]
-    m2l_c = [l for l in m2l if coarse(2 * S1 * (1 << (l - 1)))]
+    m2m_c = [l for l in m2m if 2 * S1 * (1 << l) < rows]  # 2 (P-1) planes
+    m2l_c = [l for l in m2l if 2 * S1 * (1 << (l - 1)) < rows]
     tile = max(1, 2048 // P)  # points per sections tile; S2M is fused there for whole boxes
     fused = tile % b == 0 and T % 4 == 0
     return {
@@ -786,7 +791,7 @@ def main():
     if rank == 0:
         ms_step = tot / K
         value = replicas.whole_job_rate(N, K, world, tot) / 1e6
-        byts = stage_bytes(N, P, T, b, esz)
+        byts = stage_bytes(N, P, T, b, esz, coarse_rows(plan.describe()))
         hbm, peak_kind = peaks()
         stage_tab = {}
         for name, (ms, launches) in stages.items():

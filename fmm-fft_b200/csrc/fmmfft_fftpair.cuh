@@ -147,7 +147,7 @@ struct CombineLd2 : CombineLd<float> { /* columns m, m + 1 (even m: 8-byte loads
 
 /* Blocks of 512 threads, two an SM, also ask L2 for the input of the block that follows in their place
  * (2^24, P = 64: passes 72 / 63 us -> 70 / 59). */
-constexpr unsigned kPairAhead = 2 * 148;
+constexpr unsigned kPairAhead = 2 * 148; /* a distance only: on another number of SMs a block asks too early or late */
 
 /* L = 2^LGT (LGT = 0: any); q L / 8 threads a pair of sequences, W / 2 pairs a block.  TIN and TOUT as in
  * k_fft_reg. */

@@ -12,9 +12,9 @@
  *   4  M2M             row contraction per level: phi_L = [phi_L+1 pair] . [S_L;S_R]  (:476-515)
  *   5  top flip        psi_2[c] = topflp . phi_2[c+2]                    (:620-639)
  *   6  M2L + L2L       row contraction per level over parent boxes, both children at once
- *                      (:643-749); the tree levels of stages 4-6 with few rows (FP64 under
- *                      1024, FP32 under 2048; at most 64 boxes per plane) run in one launch,
- *                      k_coarse, a block per plane
+ *                      (:643-749); the tree levels of stages 4-6 with few rows (under 1024 in
+ *                      FP64 and 2048 in FP32 where the row contractions take the rest, else under
+ *                      4096; at most 64 boxes per plane) run in one launch, k_coarse, a block per plane
  *   7  leaf            row contraction per section: u = [psi_n | x window] . [E_sc ; cot
  *                      Toeplitz] with the half-shifted first point as one more operator column
  *                      (tensor cores) + k_leaf_mid for section P/2; row contractions for FP32 /
@@ -28,7 +28,8 @@
  *                      shapes they do not take) (FFTW at :1080)
  *  10  k_block_dc      FP32 plans: the block-DC bins from the exact identity in FP64
  *
- * Sections of up to a few thousand points run stages 1 to 7 in one block each (fmmfft_tree.cuh).  Row
+ * Sections of up to a few thousand points run stages 1 to 7 in one block each, where the device holds all
+ * of a transform's at once (fmmfft_tree.cuh, tree_setup).  Row
  * contractions: FP64 on the FP64 matrix instructions (fmmfft_rows.cuh), FP32 on the CUDA cores
  * (fmmfft_rows32.cuh), split-TF32 and BF16x3 plans on tcgen05 where rows are long and levels large
  * (fmmfft_tc.cuh, the leaf fmmfft_tcss.cuh) and as FP32 otherwise; rowgemm for shapes these do not take.
@@ -184,7 +185,7 @@ template <typename R> struct Dev {
   int ss_leaf;      /* stages of the leaf's shared-memory form (tc::k_tc_ss), 0: not used */
   int kp_s2m, np_s2m, kp_m2m, np_m2m, kp_m2l, np_m2l, kp_leaf, np_leaf;
   int ok_s2m, ok_m2m, ok_m2l, ok_leaf;
-  int kp_lnb, np_lnb, ok_lnb; /* neighbour-sum leaf (tc::k_tc_nbr): the leaf's default form */
+  int kp_lnb, np_lnb, ok_lnb; /* neighbour-sum leaf (tc::k_tc_nbr): sections of under 128 boxes */
   long tc_min_rows; /* stages with fewer rows use the CUDA-core kernel */
   int fft_threads;  /* threads per block of the register FFT pass (power of two, <= 512) */
   /* tensor-core kernel: 0 row form (32 lanes), 3 row form (16 lanes), 4 warp-specialised; -1
@@ -195,7 +196,6 @@ template <typename R> struct Dev {
   int form_m2l; /* M2L's tensor-core form when tc_form does not force one */
   int bf16;    /* FMMFFT_BF16X3: the tensor-core stages in BF16x3 instead of split TF32 */
   int pdl;     /* row-form launches as programmatic dependent launches (FMMFFT_PDL=0: off) */
-  unsigned *sync;   /* grid barrier of the coarse-tree kernel: [0] arrivals, [32] generation */
   long coarse_rows; /* levels with fewer rows go to the coarse-tree kernel (0: none) */
   int coarse_grid;  /* blocks of the coarse-tree kernel an SM holds (0: its operators do not fit) */
   int fuse_s2m;     /* S2M inside the sections pass where tiles hold whole boxes */
@@ -2378,8 +2378,8 @@ template <typename R> static int tc_upload_ops(Dev<R> *d, const fmm_ops64 *o, ch
   return rc;
 }
 
-constexpr long kRowsMinRows = 1024; /* the same with the row contractions of fmmfft_rows.cuh, fmmfft_rows32.cuh */
 constexpr long kCoarseRows = 4096; /* default: tree levels with fewer rows form the coarse tree */
+constexpr long kRowsMinRows = 1024; /* where the row contractions take the other levels: FP64, twice that in FP32 */
 
 /* Coarse-tree settings of a plan: threshold (FMMFFT_COARSE_ROWS overrides, 0 turns the
  * one-launch coarse tree off) and whether the kernel's shared memory fits.  The choice depends on
@@ -2602,7 +2602,6 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
   CARVE(z, nb * P * M, C)
   CARVE(tmp, nb * P * M, C)
   CARVE(status, 1, int)
-  CARVE(sync, 64, unsigned)
   CARVE(tcs2m, 2 * sz_s2m, float)
   CARVE(tcm2m, 2 * sz_m2m, float)
   CARVE(tcm2l, 2 * sz_m2l, float)
@@ -2660,7 +2659,6 @@ static int dev_create(const fmm_ops64 *o, int precision, int nb, Dev<R> **out, c
   d->tmp = (C *)(base + off_tmp);
   d->u = (R *)(base + off_u);
   d->status = (int *)(base + off_status);
-  d->sync = (unsigned *)(base + off_sync);
   d->tc_s2m[0] = (float *)(base + off_tcs2m), d->tc_s2m[1] = (float *)(base + off_tcs2m16);
   d->tc_m2m[0] = (float *)(base + off_tcm2m), d->tc_m2m[1] = (float *)(base + off_tcm2m16);
   d->tc_m2l[0] = (float *)(base + off_tcm2l), d->tc_m2l[1] = (float *)(base + off_tcm2l16);
@@ -3837,7 +3835,7 @@ static float g_noalloc_stage[FMMK_NOALLOC_STAGE_FLOATS];
  * complex64 plan (dev_create), offsets relative to the array base. */
 struct NoallocLayout {
   size_t initch, btop, bm2m, bm2l, evalmT, evalmh, cot, pretw, twP, twM, xt, part, ssum, phi, psi,
-      u, z, tmp, sync, end;
+      u, z, tmp, status, end;
 };
 
 static NoallocLayout noalloc_layout(const fmm_ops64 *o, long ntile) {
@@ -3869,7 +3867,7 @@ static NoallocLayout noalloc_layout(const fmm_ops64 *o, long ntile) {
   L.u = take(sizeof(float) * 2 * S1 * M);
   L.z = take(sizeof(float2) * P * M);
   L.tmp = take(sizeof(float2) * P * M);
-  L.sync = take(64 * sizeof(unsigned));
+  L.status = take(sizeof(int));
   L.end = off;
   return L;
 }
@@ -3958,13 +3956,13 @@ extern "C" int fmmk_execute_noalloc(const fmm_ops64 *o, int reuse_ops, const voi
   d.M = o->M, d.P = o->P, d.T = o->T, d.b = o->b, d.s = o->s, d.n = o->n;
   d.N = o->M * o->P, d.S1 = o->P - 1, d.precision = 1;
   d.fft_threads = 512;
-  /* the same stage choices as an FMMFFT_F32 plan (dev_create), including its switches */
+  /* FP32 on the general stage kernels, one launch a level: k_rowgemm, k_leaf, the paired FFT passes.  The
+   * array has no place for the operators of the row contractions, whole sections and coarse levels that an
+   * FMMFFT_F32 plan takes, so its sums run in another order (both within 1e-6 of the FP64 transform). */
   d.fuse_s2m = 1;
   if (const char *ev = getenv("FMMFFT_FUSE_S2M")) d.fuse_s2m = atoi(ev) != 0;
   d.pdl = 1;
   if (const char *ev = getenv("FMMFFT_PDL")) d.pdl = atoi(ev) != 0;
-  /* no cooperative coarse-tree kernel here: a timeout of its grid barrier could not be
-   * reported by this entry point (sizes it serves never reach the coarse-tree threshold) */
   d.coarse_rows = 0;
   d.tileM = d.P >= 2048 ? 1 : 2048 / d.P;
   if (d.tileM > d.M) d.tileM = d.M;
@@ -4016,8 +4014,7 @@ extern "C" int fmmk_execute_noalloc(const fmm_ops64 *o, int reuse_ops, const voi
   d.u = (float *)(base + L.u);
   d.z = (float2 *)(base + L.z);
   d.tmp = (float2 *)(base + L.tmp);
-  d.sync = (unsigned *)(base + L.sync);
-  d.status = (int *)(d.sync + 48); /* the coarse-tree barrier records a timeout here */
+  d.status = (int *)(base + L.status); /* no kernel of this entry waits, so none writes it */
   d.nbmax = 1;
   return dev_execute<float>(&d, d_in, d_out, st, 0, 1, err, errlen);
 }
@@ -4281,7 +4278,7 @@ extern "C" void fmmk_batch_free(void *exec) {
 /* ======================================================================== plain size-N FFT */
 
 /* A conventional FFT of the whole N-vector on the GPU, the same register Stockham passes as the
- * FMM-FFT's size-M FFTs: one pass (N <= 4096), a 4-step of two passes (N <= 2^21) or a 4-step
+ * FMM-FFT's size-M FFTs: one pass (N <= 4096), a 4-step of two passes (N <= 2^22) or a 4-step
  * whose second factor is itself a 4-step (three passes, N <= 2^30).  It stands where the
  * reference's plain FFTW comparators stand (src/fftw_serial.c:53-58, src/fftw_mpi.c:54-58):
  * FMM-FFT against an ordinary FFT of the same length on the same machine.  Forward,
@@ -4333,8 +4330,8 @@ extern "C" int fmmk_fft_create(long N, int dbl, fmmk_fft **out, size_t *device_b
     f->pass[0] = plain_pass((int)N, 1, N, N, 1, N, N, 1, 0, 1, N);
     f->per[0] = 1, f->rows[0] = 1, f->tin[0] = 1, f->tout[0] = 1, f->src[0] = 0, f->dst[0] = 1;
   } else if (lg <= 22) {
-    /* Two passes while both lengths stay at 2^11: a block then has 4 sequences, 32-byte pieces, which cost less
-     * than a third pass (2^22, us: FP32 79 -> 65, FP64 161 -> 142).  Below 2^21 a first pass of at most 2^9, so that its
+    /* Two passes while both lengths stay at 2^11: a block then has 4 sequences (FP64 2), 32-byte pieces, which cost
+     * less than a third pass (2^22, us: FP32 79 -> 65, FP64 161 -> 142).  Below 2^21 a first pass of at most 2^9, so that its
      * pieces are longer (FP64 2^20: 40, with 2^10 42; 2^21 85, with 2^10 77). */
     const int a = lg >= 21 || lg / 2 <= 9 ? lg / 2 : 9;
     const long N2 = 1L << a, N1 = N / N2;

@@ -21,7 +21,7 @@
  *
  * Measured, neighbour-sum form -> this one (us a leaf): 2^20 P64 T20 31 -> 24, 2^22 P64 T8 66 -> 50,
  * 2^24 P64 T24 234 -> 197, 2^26 P256 T16 860 -> 648 (b = 32).  The small A_lo products enter the
- * accumulator while it is small: relative L2 error of the transform 2.9e-7 -> 2.1e-7.  What bounds it:
+ * accumulator while it is small: relative L2 error of the transform at 2^26 2.9e-7 -> 2.4e-7.  What bounds it:
  * 60% of a tile's 7 k cycles are the MMAs, about 130 cycles each where both operands (7 KB) come from
  * shared memory; the rest is producers and epilogue that share that memory's bandwidth with them.
  * M2M, S2M and M2L in this form were slower than rows of 16 lanes (2^24: 158 against 109, .., 286 / 217).

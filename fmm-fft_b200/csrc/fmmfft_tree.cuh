@@ -4,7 +4,7 @@
  *
  * Every section of the transform is a tree of its own from its samples to its field, so sections of
  * up to a few thousand points need no launch between levels, no planar copy of the samples and no
- * pass for their sums.  Here a stage costs two
+ * pass for their sums; which plans take it is tree_setup's rule.  Here a stage costs two
  * block barriers, and its contraction is blk_gemm: out[row][c] = sum_k A(row, k) B[k][c], A rows and B
  * in shared memory, a thread (FP32) a register tile of the output, a warp (FP64) tiles of the FP64
  * matrix instruction.  Bound by latency: a stage of a small section is a chain of a few hundred

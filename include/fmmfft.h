@@ -99,8 +99,8 @@ void mft(long lq, void *qr, long dir, long p, long myid, long terms, long b, dou
  * with FMMFFT_ERR_TIMEOUT and its block untouched.  Calls with mismatched (lq, p, terms, b) or
  * a repeated myid are refused.  fmmfft_mft_rank_mode(0) restores full-vector calls; switching
  * is refused with FMMFFT_ERR_BUSY while a collective is in progress.  MPI callers whose ranks
- * are processes gather the blocks to one rank and call fmmfft_execute_blocks_host there
- * (INTEGRATION.md shows the binding). */
+ * are processes gather the blocks to one rank, call fmmfft_execute_blocks_host there and scatter
+ * the results. */
 int fmmfft_mft_rank_mode(int on);
 
 /* Status of the calling thread's last compatibility call (FMMFFT_OK after success). */
@@ -122,7 +122,11 @@ int fmmfft_plan_destroy(fmmfft_plan plan);
  * threshold and the fused S2M are timed and the fastest kept; later plans of that key take the
  * same choice (so they compute the same bits).  FMMFFT_AUTOTUNE=0 keeps the defaults; a knob
  * set by its environment switch is not tuned.  fmmfft_plan_describe writes the plan's choices
- * as text ("fft_threads=512 coarse_rows=4096 ..."). */
+ * as text ("fft_threads=512 coarse_rows=4096 ... s2m=rows ..."); 256 characters hold it.  Some switches
+ * also take the plan off its newer kernels: FMMFFT_COARSE_ROWS and FMMFFT_FUSE_S2M set to any value keep
+ * every stage on the general and tensor-core stage kernels (no sections whole in one block, no row
+ * contractions); FMMFFT_TC_FORM, _TC_MIN_ROWS, _TC_STAGES and _LEAF_FORM do so on tensor-core plans, the
+ * shared-operand leaf included, and on other plans turn off sections whole in one block. */
 int fmmfft_plan_describe(fmmfft_plan plan, char *buf, size_t len);
 /* Device bytes the plan holds (operators + workspace). */
 int fmmfft_plan_device_bytes(fmmfft_plan plan, size_t *bytes);
@@ -320,9 +324,9 @@ const char *fmmfft_stage_name(int i);
 /* ------------------------------------------------------------------ allocation-free entry */
 /* No counterpart in the reference.  For callers that cannot call cudaMalloc: code that runs
  * under a device-memory budget owned by someone else (a pool or arena it may not grow), or in a
- * phase where it must not allocate at all.  Forward transform of N complex64 values (FP32, the
- * FMMFFT_F32 arithmetic, same result as fmmfft_execute on an FMMFFT_F32 plan) from d_in to
- * d_out, both caller-owned device buffers, enqueued on `stream`.  Nothing is allocated: the
+ * phase where it must not allocate at all.  Forward transform of N complex64 values (FP32, as
+ * accurate as fmmfft_execute on an FMMFFT_F32 plan, on the general stage kernels: other sums, so other
+ * last bits, and a launch a level) from d_in to d_out, both caller-owned device buffers, enqueued on `stream`.  Nothing is allocated: the
  * operator tables and the workspace live in one file-scope device array of 32 MiB that every
  * GPU which loads this library holds until process exit (the FP64 operator build uses a
  * file-scope 16 MiB host array).  Sizes whose tables plus workspace exceed 32 MiB (about
