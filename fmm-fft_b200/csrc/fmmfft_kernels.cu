@@ -2404,17 +2404,19 @@ template <typename R> static void coarse_setup(Dev<R> *d) {
 /* Whether the plan's sections run whole in one block (k_tree).  FP64 plans: up to 1024 points a section
  * (16 terms: 16 of 2^16 144 us in one block / 232 in stages, 16 of 2^17 345 / 308, where the row contractions
  * fill the device).  FP32 plans of every kind: where the sections of one transform, P blocks, are on the
- * device at once, with twice as many where the stages lack the FP32 row contractions for their large levels
- * (more than 32 terms; BF16x3), and above 512 sections only up to 32 points each.  More sections than
+ * device at once, above 512 sections only up to 32 points each; twice as many sections of any number with 33
+ * to 44 terms, for which the stages have no row contractions (with more terms a level's operator is most of a
+ * block's memory and time: 16 transforms of P = 256, 128 points, 64 terms 467 us / 326 in stages).  More sections than
  * that lose to the stages, alone and in a batch (us, one block / stages, split TF32, b = 32: P = 512 of 4096
  * points, 24 terms 402 / 179; P = 256 of 4096, 16 terms, 4 transforms 545 / 234; P = 1024 of 256, 24 terms, 16
  * transforms 614 / 441); fewer win alone (P = 64 of 1024, 20 terms 39 / 45).  Over 1550 shapes and
- * batches the rule's transforms take 0.92 of the time of one block wherever it fits, none more than when
- * there were only stages.  The choice depends on the shape alone, so that a transform takes the same kernel
+ * batches of up to 33 terms the rule's transforms take 0.92 of the time of one block wherever it fits, none
+ * more than when there were only stages.  The choice depends on the shape alone, so that a transform takes the same kernel
  * alone and in a batch.  A switch that steers the stage kernels keeps those. */
 constexpr long kTreeMaxF64 = 1024, kTreeSms = 148; /* SMs of the device: a constant, a shape's route is fixed */
-static bool tree_one_wave(long M, long P, int blocks, bool no_rows) {
-  return P > 512 ? M <= 32 : P <= kTreeSms * blocks * (no_rows ? 2 : 1);
+static bool tree_one_wave(long M, long P, long T, int blocks) {
+  if (T > 32 && T <= 44) return P <= 2 * kTreeSms * blocks;
+  return P > 512 ? M <= 32 : P <= kTreeSms * blocks;
 }
 template <typename R> static void tree_setup(Dev<R> *d) {
   using E = typename TreeEng<R>::E;
@@ -2423,9 +2425,13 @@ template <typename R> static void tree_setup(Dev<R> *d) {
   /* blocks of 128 threads that an SM holds: by shared memory, at most the five that registers allow */
   const size_t sm = tree_smem<E>(T, b, n, 0) + 1024;
   d->tree_blocks = sm * 5 <= (size_t)227 * 1024 ? 5 : (int)((size_t)227 * 1024 / sm);
-  d->tree = b >= 8 && b <= 64 && (sizeof(R) == 4 ? tree_one_wave(d->M, d->P, d->tree_blocks, T > 32 || d->bf16) : d->M <= kTreeMaxF64) &&
+  const bool fits = b >= 8 && b <= 64 && (sizeof(R) == 4 || d->M <= kTreeMaxF64) &&
             !(d->env_set & (KNOB_COARSE | KNOB_TCMIN | KNOB_FUSE | KNOB_FORM)) && !getenv("FMMFFT_TC_STAGES") &&
             !getenv("FMMFFT_LEAF_FORM") && tree_smem<E>(T, b, n, 0) <= (size_t)200 * 1024;
+  d->tree = fits && (sizeof(R) == 8 || tree_one_wave(d->M, d->P, T, d->tree_blocks) || (d->bf16 && !d->rows));
+  /* a BF16x3 plan computes sections of these sizes in FP32 in its stages too, which is no slower (2^20, P = 256, 16
+   * terms, b = 16, us: in one block 126, FP32 stages 112, BF16x3 stages 146) */
+  if (d->bf16 && fits && !d->tree) d->ok_s2m = d->ok_m2m = d->ok_m2l = d->ok_leaf = d->ok_lnb = d->ss_leaf = 0;
 }
 
 static void rows_smem_limits(int T, int b);
