@@ -284,15 +284,15 @@ template <class E> struct TreeArgs {
   InTab xin;
 };
 
-/* Values of the largest operator, and of the operators' place in shared memory */
-template <class E> __host__ __device__ __forceinline__ int tree_opn(int T, int b) {
-  int m = 8 * tree_blk<E>(T);
+/* Values of the largest operator (M2L's where there is one), and of the operators' place in shared memory */
+template <class E> __host__ __device__ __forceinline__ int tree_opn(int T, int b, int n) {
+  int m = (n > 2 ? 8 : 1) * tree_blk<E>(T);
   if (tree_nleaf<E>(T, b) > m) m = tree_nleaf<E>(T, b);
   if (b * E::npad(T) > m) m = b * E::npad(T);
   return m;
 }
 template <class E> __host__ __device__ __forceinline__ int tree_op_area(int T, int b, int n, int resident) {
-  return resident ? b * E::npad(T) + (10 * (n - 2) + 1) * tree_blk<E>(T) + tree_nleaf<E>(T, b) : tree_opn<E>(T, b);
+  return resident ? b * E::npad(T) + (10 * (n - 2) + 1) * tree_blk<E>(T) + tree_nleaf<E>(T, b) : tree_opn<E>(T, b, n);
 }
 constexpr int kTreeMaxLevel = 12;                             /* n <= 12 */
 constexpr int kTreeStages = 2 * (kTreeMaxLevel - 2) + 3; /* S2M, M2M n-1 .. 2, top flip, M2L 3 .. n, leaf */

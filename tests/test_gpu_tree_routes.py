@@ -26,7 +26,7 @@ def fm():
 @pytest.mark.parametrize("M,P,T,b,prec,one_block", [
     (4096, 512, 24, 32, "f32_tc", False), (2048, 512, 24, 16, "f32", False), (1024, 512, 16, 32, "f32_tc", True),
     (4096, 256, 24, 32, "f32_tc", False), (4096, 256, 16, 16, "bf16x3", False), (2048, 256, 16, 32, "f32", True),
-    (256, 1024, 33, 32, "f32_tc", True), (256, 1024, 40, 64, "f32", False), (128, 256, 64, 16, "f32", False), (128, 128, 64, 16, "f32_tc", True),
+    (256, 1024, 33, 32, "f32_tc", True), (256, 1024, 40, 64, "f32", False), (128, 256, 64, 16, "f32", False), (128, 128, 64, 16, "f32_tc", True), (64, 256, 64, 16, "f32", True),
     (4096, 128, 24, 32, "f32_tc", True), (8192, 64, 16, 64, "f32", True), (2048, 256, 33, 32, "f32_tc", True),
     (64, 1024, 8, 8, "f32_tc", False), (256, 1024, 24, 32, "f32_tc", False), (32, 1024, 12, 8, "f32", True),
     (1024, 1024, 8, 32, "f64", True), (2048, 64, 8, 32, "f64", False)])
